@@ -9,6 +9,17 @@
 
 namespace b200attn {
 
+// One thread of a fully active warp, the same one on every call.  tcgen05 and bulk-tensor instructions take their
+// descriptors and addresses from uniform registers: in a branch that the compiler knows to be taken by one thread it
+// computes them there, whereas under `lane == 0` it moves every operand over from the vector registers first
+// (MMAs of M = 128, N = 64 / 128 / 256 issued back to back on B200: 72 / 72 / 128 clocks each under `lane == 0`,
+// 49 / 64 / 128 under elect.sync).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 // ---- cluster ------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
