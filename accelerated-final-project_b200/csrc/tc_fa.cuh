@@ -814,13 +814,9 @@ inline int fa_encode_copies(const b200attn_args &a, int rd, float base, T *q_cop
     rp.cos_cache = rp.sinus ? nullptr : a.cos_cache;
     rp.sin_cache = rp.sinus ? nullptr : a.sin_cache;
     rp.X = a.Q; rp.Y = q_copy; rp.L = a.len_q;
+    if (pe_encodes_k(a.pe)) { rp.X2 = a.K; rp.Y2 = k_copy; rp.L2 = a.len_k; }
     cudaError_t e = launch_rope_k<T>(rp, sm_count, st);
     launches->fetch_add(1);
-    if (e == cudaSuccess && pe_encodes_k(a.pe)) {
-        rp.X = a.K; rp.Y = k_copy; rp.L = a.len_k;
-        e = launch_rope_k<T>(rp, sm_count, st);
-        launches->fetch_add(1);
-    }
     if (e != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "encoding kernel launch failed: %s", cudaGetErrorString(e)); return B200ATTN_ERR_CUDA; }
     *b = a;
     b->Q = q_copy;

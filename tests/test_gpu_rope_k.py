@@ -92,3 +92,20 @@ def test_caller_supplied_caches_on_the_tensor_core_path(pkg, cuda, pe):
     assert pkg.last_path() == "tc_wide"
     err = float(np.abs(got - want).max())
     assert err <= 8e-3, err
+
+
+@pytest.mark.parametrize("half", [0, 1])
+@pytest.mark.parametrize("heads", [1, 4, 5, 37])
+def test_rotation_of_many_heads_is_the_rotation_of_each(pkg, cuda, heads, half):
+    """The heads are shared out over the grid, four in flight per thread: every head of a call, whole rounds and
+    remainders, has the bits of a call on that head alone."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(heads)
+    for dtype, L, D, rd in ((torch.bfloat16, 77, 64, 32), (torch.float32, 1000, 64, 64)):
+        x = torch.randn((1, heads, L, D), generator=g, device=cuda).to(dtype)
+        pairing = pkg.PE_ROPE_HALF if half else pkg.PE_ROPE_INTERLEAVED
+        got = pkg.rope_k(x, pairing=pairing, rotary_dim=rd)
+        for h in range(heads):
+            one = pkg.rope_k(x[:, h:h + 1].contiguous(), pairing=pairing, rotary_dim=rd)
+            assert torch.equal(got[:, h:h + 1], one), (dtype, h)
