@@ -206,3 +206,27 @@ def test_fused_path_very_long_keys(pkg, cuda):
     got = run(pkg, cuda, bits)
     assert pkg.last_path() == "tc_fused"
     assert float(np.abs(got - ol.attention(*up)).max()) <= 8e-3
+
+
+@pytest.mark.parametrize("D", [8, 40, 72, 80, 96, 104, 136, 160, 192, 200, 248])
+@pytest.mark.parametrize("lens", [(130, 300), (300, 129), (3, 200)], ids=str)
+def test_widths_between_the_column_groups(pkg, cuda, D, lens):
+    """Any multiple of 8: widths whose last 16-column step is half empty (8, 40, 72, 104, ...), whose last 64-column group is
+    short, and a whole number of groups that is not a power of two (192); a few queries too where no other tensor-core
+    path takes the width.  Nothing behind the output is written."""
+    import torch
+    (Lq, Lk), B, H = lens, 1, 3
+    bits, up = bf16_problem(B, H, Lq, Lk, D, 100 + D, "normal")
+    want = ol.attention(*up)
+    q, k, v = (bf16_to_dev(b, cuda) for b in bits)
+    big = torch.full((B * H * Lq * D + 256,), 3.0, dtype=torch.bfloat16, device=cuda)
+    out = big[:B * H * Lq * D].view(B, H, Lq, D)
+    pkg.forward(q, k, v, out=out)
+    assert pkg.last_path() == ("tc_wide" if D == 192 and Lq <= 64 else "tc_fused"), pkg.last_path()
+    assert bool((big[B * H * Lq * D:] == 3.0).all())
+    assert float(np.abs(bf16_from_dev(out) - want).max()) <= 8e-3   # the bound of the whole widths: P and the result rounded to bf16
+    got = pkg.forward(*(t.to(torch.float16) for t in (q, k, v)))
+    assert float(np.abs(got.float().cpu().numpy() - want).max()) <= 4e-3   # fp16: the suite's bound
+    if D % 16 == 0:
+        got = run(pkg, cuda, bits, pe=pkg.PE_ROPE_INTERLEAVED)
+        assert float(np.abs(got - ol.attention(*up, pe=ol.PE_ROPE_INTERLEAVED)).max()) <= TOL
