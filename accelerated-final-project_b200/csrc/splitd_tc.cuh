@@ -260,7 +260,7 @@ sdtc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     grid_launch_dependents();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- the buffer of the scratch ring is clean once its earlier users have cleared their heads ----
             unsigned seen = 0;
             for (unsigned it = 0; it < lim; ++it) {
@@ -305,7 +305,7 @@ sdtc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- score MMAs: per 8 columns two M = 64, N = 128 MMAs into one accumulator, Q hi [K hi; K lo]^T and
             // Q lo [K hi; K lo]^T: a row's products with K hi in columns 0-63, with K lo in columns 64-127 ----
             const uint32_t id = umma_idesc_tf32(64, 128, 0, 0);
@@ -492,7 +492,7 @@ sdtc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         ST_DBG(3, if (h == 0 && threadIdx.x < 64) { p.dbg[512 + threadIdx.x] = reinterpret_cast<float *>(p_buf)[threadIdx.x]; p.dbg[576 + threadIdx.x] = reinterpret_cast<float *>(v_hi)[threadIdx.x];
                                                     p.dbg[640 + threadIdx.x] = reinterpret_cast<float *>(v_lo)[threadIdx.x]; });
         if (threadIdx.x == 0) ST_STAMP(h == 0 ? 11 : 27);
-        if (warp == 1 && lane == 0 && !failed) {
+        if (warp == 1 && !failed && elect_one()) {
             const uint32_t idv = umma_idesc_tf32(128, 128, 1, 0);
             for (int kk = h * kpc; kk < ksteps && kk < (h + 1) * kpc; ++kk) {
                 const int kl = kk - h * kpc;

@@ -192,7 +192,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
     } else if (warp < 4) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FA_REGS_SMALL));
       if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;            // ring stage and the parity of its use (kept by hand: a division here costs the thread hundreds of clocks)
             uint32_t ph = 0;
             int ui = 0;
@@ -223,7 +223,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
             TC_PROF_FLUSH(8, true);
         }
       } else if (warp < 3) {
-        if (lane == 0) {
+        if (elect_one()) {
             const int t = warp - 1;
             const uint32_t id_qk = umma_idesc_16(FA_BM, FA_BN, 0, 0, F16 ? 1 : 0), id_pv = umma_idesc_16(FA_BM, 16 * ks, 0, 1, F16 ? 1 : 0);
             const uint32_t qa = smem_u32(q_smem + (size_t)t * tile_bytes), pa = smem_u32(p_smem + (size_t)t * FA_P_BYTES);
@@ -480,7 +480,7 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     if (skip) {
         // fall through to the common exit
     } else if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;            // ring stage and the parity of its use (kept by hand: a division here costs the thread hundreds of clocks)
             uint32_t ph = 0;
             int ui = 0;
@@ -519,7 +519,7 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
             if (!ok) { report_kernel_error(p.err, p.err_sys, (unsigned)KERR_MBAR_TIMEOUT | (1u << 7)); failed = true; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t id_qk = umma_idesc_16(FA_BM, FA_BN, 0, 0, F16 ? 1 : 0), id_pv = umma_idesc_16(FA_BM, 16 * ks, 0, 1, F16 ? 1 : 0);
             int s = 0;                  // ring stage and the parity of its use
             uint32_t ph = 0;
