@@ -18,6 +18,7 @@
 #include "../../include/b200attn.h"
 #include "splitd.cuh"
 #include "splitd_tc.cuh"
+#include "splitd_stream.cuh"
 #include "rope_k.cuh"
 #include "synth.cuh"
 #include "tc_bf16.cuh"
@@ -59,20 +60,20 @@ struct TmapCache {
         CUtensorMap map;
         const void *base = nullptr;
         long long rows = 0;
-        int cols = 0, box_rows = 0, swz = 0;
+        int cols = 0, box_rows = 0, swz = 0, esz = 0;
         bool valid = false;
     };
     static constexpr size_t kEntries = 4096;   // direct-mapped
     std::vector<Entry> e;
-    // fp32 [rows][cols] matrix, box [box_rows x 32 columns], one of the 128-byte swizzles
-    const CUtensorMap *get(const void *base, long long rows, int cols, int box_rows, CUtensorMapSwizzle swz) {
+    // [rows][cols] matrix of fp32 (esz 4) or 16-bit (2) elements, box [box_rows x 32 columns]
+    const CUtensorMap *get(const void *base, long long rows, int cols, int box_rows, CUtensorMapSwizzle swz, int esz = 4) {
         if (e.empty()) e.resize(kEntries);
         size_t h = (size_t)((uintptr_t)base >> 4) * 0x9E3779B97F4A7C15ull;
-        h ^= (size_t)rows * 0xC2B2AE3D27D4EB4Full + (size_t)cols * 1315423911u + (size_t)box_rows + ((size_t)swz << 40);
+        h ^= (size_t)rows * 0xC2B2AE3D27D4EB4Full + (size_t)cols * 1315423911u + (size_t)box_rows + ((size_t)swz << 40) + ((size_t)esz << 48);
         Entry &x = e[(h >> 20) % kEntries];
-        if (!(x.valid && x.base == base && x.rows == rows && x.cols == cols && x.box_rows == box_rows && x.swz == (int)swz)) {
-            x.valid = make_tmap_2d(&x.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, ST_ATOM, box_rows, swz);
-            x.base = base; x.rows = rows; x.cols = cols; x.box_rows = box_rows; x.swz = (int)swz;
+        if (!(x.valid && x.base == base && x.rows == rows && x.cols == cols && x.box_rows == box_rows && x.swz == (int)swz && x.esz == esz)) {
+            x.valid = make_tmap_2d(&x.map, esz == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, esz, base, rows, cols, ST_ATOM, box_rows, swz);
+            x.base = base; x.rows = rows; x.cols = cols; x.box_rows = box_rows; x.swz = (int)swz; x.esz = esz;
             if (!x.valid) return nullptr;
         }
         return &x.map;
@@ -110,6 +111,8 @@ struct DeviceCtx {
     unsigned sdtc_seq = 0;         // calls so far: call n uses buffer n % ST_NBUF
     unsigned sdtc_gen_expect[ST_NBUF] = {};   // heads the earlier users of each buffer will have cleared
     bool sdtc_attr = false;
+    bool sw_attr = false;
+    SwTables sw_tables;            // angles of the streamed split-head_d kernel
     size_t sdtc_smem_max = 0;
     // the last enqueued call, when it was this kernel: a following call that is declared independent of it
     // (b200attn_forward_many) may be launched as its programmatic dependent
@@ -355,6 +358,19 @@ static int run_splitd(DeviceCtx &c, const b200attn_args &a, int rd, float base, 
     return B200ATTN_OK;
 }
 
+// the score-scratch ring of the tensor-core split-head_d kernels
+static int ensure_ring(DeviceCtx &c, cudaStream_t st) {
+    if (c.sdtc_S == nullptr) {
+        const int cap = c.sm_count;
+        CU_TRY(cudaMalloc(&c.sdtc_S, (size_t)ST_NBUF * cap * 4096 * sizeof(float)));
+        CU_TRY(cudaMalloc(&c.sdtc_cnt, (size_t)ST_NBUF * cap * 2 * sizeof(unsigned)));
+        CU_TRY(cudaMalloc(&c.sdtc_gen, ST_NBUF * sizeof(unsigned)));
+        c.sdtc_cap = cap;
+        c.scratch_dirty = true;   // cleared below, on this call's stream
+    }
+    return c.scratch_dirty ? ensure_scratch(c, 0, 0, st) : B200ATTN_OK;
+}
+
 #ifdef B200ATTN_DEVTOOLS
 static float *g_sdtc_dbg = nullptr;
 static unsigned long long *g_sdtc_stamps = nullptr;
@@ -438,18 +454,7 @@ static int run_sdtc(DeviceCtx &c, const b200attn_args &a, cudaStream_t st, bool 
         c.sdtc_attr = true;
     }
     if (smem > c.sdtc_smem_max) return -1;
-    if (c.sdtc_S == nullptr) {
-        const int cap = c.sm_count;
-        CU_TRY(cudaMalloc(&c.sdtc_S, (size_t)ST_NBUF * cap * 4096 * sizeof(float)));
-        CU_TRY(cudaMalloc(&c.sdtc_cnt, (size_t)ST_NBUF * cap * 2 * sizeof(unsigned)));
-        CU_TRY(cudaMalloc(&c.sdtc_gen, ST_NBUF * sizeof(unsigned)));
-        c.sdtc_cap = cap;
-        c.scratch_dirty = true;   // cleared below, on this call's stream
-    }
-    if (c.scratch_dirty) {
-        int rc = ensure_scratch(c, 0, 0, st);
-        if (rc) return rc;
-    }
+    if (int rc = ensure_ring(c, st)) return rc;
     // (the four maps are copied before the next lookup can evict one: the cache is direct-mapped)
     CUtensorMap tmQ, tmK, tmV;
     const CUtensorMap *m;
@@ -496,6 +501,82 @@ static int run_sdtc(DeviceCtx &c, const b200attn_args &a, cudaStream_t st, bool 
     c.prev_out_hi = (uintptr_t)a.out + in_q;
     g_launches.fetch_add(1);
     t_last_path = "splitd_tc";
+    return B200ATTN_OK;
+}
+
+// ---- the same with streamed slices (splitd_stream.cuh): wide slices, 16-bit tensors, encodings of neighbouring columns -----
+static bool sw_supported(const DeviceCtx &c, const b200attn_args &a) {
+    if (a.len_q > 64 || a.len_k > 64) return false;
+    const int esz = a.dtype == B200ATTN_F32 ? 4 : 2;
+    if (a.head_d % (16 / esz) != 0) return false;   // rows of whole 16-byte units: what a tensor map describes
+    if (a.pe != B200ATTN_PE_NONE && a.pe != B200ATTN_PE_ROPE_INTERLEAVED && a.pe != B200ATTN_PE_ROPE_Q_ONLY && a.pe != B200ATTN_PE_SINUSOIDAL) return false;
+    if (a.pe != B200ATTN_PE_NONE && a.cos_cache != nullptr) return false;
+    if ((((uintptr_t)a.Q | (uintptr_t)a.K | (uintptr_t)a.V) & 15) != 0 || ((uintptr_t)a.out & (4 * esz - 1)) != 0) return false;
+    const long long BH = (long long)a.batch_sz * a.num_heads;
+    return BH <= c.sm_count;
+}
+
+template <typename T, bool PE, int NP>
+static int launch_sw(DeviceCtx &c, const b200attn_args *a, int n, const SwParams &p, cudaStream_t st) {
+    constexpr bool W = sizeof(T) == 4;
+    SwProblems<NP> pr;
+    for (int i = 0; i < n; ++i) {
+        const long long BH = p.BH;
+        const CUtensorMapSwizzle swz = W ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE;
+        const CUtensorMap *m;
+        bool ok = (m = c.tmaps.get(a[i].Q, BH * p.Lq, p.D, p.Lq, swz, (int)sizeof(T))) != nullptr;
+        if (ok) { pr.q[i] = *m; ok = (m = c.tmaps.get(a[i].K, BH * p.Lk, p.D, p.Lk, swz, (int)sizeof(T))) != nullptr; }
+        if (ok) { pr.k[i] = *m; ok = (m = c.tmaps.get(a[i].V, BH * p.Lk, p.D, p.Lk, swz, (int)sizeof(T))) != nullptr; }
+        if (!ok) return fail(B200ATTN_ERR_CUDA, "cuTensorMapEncodeTiled failed for the streamed slices");
+        pr.v[i] = *m;
+        pr.Q[i] = a[i].Q; pr.K[i] = a[i].K; pr.V[i] = a[i].V; pr.O[i] = a[i].out;
+    }
+    CU_TRY(launch_dependent(sw_kernel<T, PE, NP>, dim3((unsigned)p.nsplit, (unsigned)(n * p.BH)), SW_THREADS, SW_SMEM, 1, st, pr, p));
+    return B200ATTN_OK;
+}
+
+// One launch for `n` (<= SW_MAXP) problems of the same form, n heads' worth of CTAs on the chip at once.  -1: not taken, nothing launched.
+static int run_sw(DeviceCtx &c, const b200attn_args *a, int n, int rd, float base, cudaStream_t st) {
+    const long long BH = (long long)a->batch_sz * a->num_heads, heads = n * BH;
+    if (heads > c.sm_count || n > SW_MAXP) return -1;
+    if (!c.sw_attr) {
+        const void *kerns[] = {(const void *)sw_kernel<float, false, 1>, (const void *)sw_kernel<float, true, 1>, (const void *)sw_kernel<float, false, SW_MAXP>,
+                               (const void *)sw_kernel<float, true, SW_MAXP>, (const void *)sw_kernel<__nv_bfloat16, false, 1>, (const void *)sw_kernel<__nv_bfloat16, true, 1>,
+                               (const void *)sw_kernel<__half, false, 1>, (const void *)sw_kernel<__half, true, 1>};
+        for (const void *k : kerns) CU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM));
+        c.sw_attr = true;
+    }
+    if (int rc = ensure_ring(c, st)) return rc;
+    SwParams p{};
+    p.BH = (int)BH; p.Lq = a->len_q; p.Lk = a->len_k; p.D = a->head_d;
+    p.natoms = (p.D + ST_ATOM - 1) / ST_ATOM;
+    const int slots = (int)(c.sm_count / heads), per = (p.natoms + slots - 1) / slots;
+    p.nsplit = (p.natoms + per - 1) / per;
+    const int buf = (int)(c.sdtc_seq % ST_NBUF);
+    p.buf = buf; p.cap_bh = c.sdtc_cap; p.gen_expect = c.sdtc_gen_expect[buf];
+    p.pe = a->pe; p.rd = rd;
+    if (a->pe != B200ATTN_PE_NONE) {
+        const bool sinus = a->pe == B200ATTN_PE_SINUSOIDAL;
+        p.tab = c.sw_tables.get(p.D, sinus ? p.D : rd, sinus ? 10000.0f : base, sinus ? 1 : 0, st, &g_launches);
+        if (p.tab == nullptr) return -1;
+    }
+    p.scale = 1.0f / sqrtf((float)p.D);
+    p.S = c.sdtc_S; p.counters = c.sdtc_cnt; p.gen = c.sdtc_gen;
+    p.err = c.err_dev; p.err_sys = c.err_host_dev;
+    p.spin_limit = current_spin_limit();
+    p.wait_extra = g_test_wait_extra.load();
+    const bool pe = a->pe != B200ATTN_PE_NONE;
+    int rc;
+    if (a->dtype == B200ATTN_F32 && n > 1) rc = pe ? launch_sw<float, true, SW_MAXP>(c, a, n, p, st) : launch_sw<float, false, SW_MAXP>(c, a, n, p, st);
+    else if (n > 1) return -1;
+    else if (a->dtype == B200ATTN_F32) rc = pe ? launch_sw<float, true, 1>(c, a, 1, p, st) : launch_sw<float, false, 1>(c, a, 1, p, st);
+    else if (a->dtype == B200ATTN_F16) rc = pe ? launch_sw<__half, true, 1>(c, a, 1, p, st) : launch_sw<__half, false, 1>(c, a, 1, p, st);
+    else rc = pe ? launch_sw<__nv_bfloat16, true, 1>(c, a, 1, p, st) : launch_sw<__nv_bfloat16, false, 1>(c, a, 1, p, st);
+    if (rc) return rc;
+    c.sdtc_seq += 1;
+    c.sdtc_gen_expect[buf] += (unsigned)heads;
+    g_launches.fetch_add(1);
+    t_last_path = "splitd_stream";
     return B200ATTN_OK;
 }
 
@@ -549,7 +630,8 @@ static int check_kernel_errors(DeviceCtx &c, cudaStream_t st, bool sync) {
     return report_kernel_errors(c, "kernel");
 }
 
-static int forward_device(const b200attn_args *a, bool independent_of_prev = false, bool batched = false) {
+// `n` > 1: the entries a[0 .. n) are independent problems that one launch may take (batch_group); -1 when it does not.
+static int forward_device(const b200attn_args *a, bool independent_of_prev = false, bool batched = false, int n = 1) {
     int rd; float base;
     int rc = validate(a, &rd, &base);
     if (rc) return rc;
@@ -574,6 +656,10 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
     }
     c->last_stream = st;
     c->have_last_stream = true;
+    if (n > 1) {
+        c->prev_sdtc = false;
+        return run_sw(*c, a, n, rd, base, st);
+    }
     bool done = false;
     const bool chain = independent_of_prev && c->prev_sdtc;
     c->prev_sdtc = false;   // set again by the kernel that supports being overlapped
@@ -644,6 +730,11 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
         if (rc != B200ATTN_OK) c->prev_sdtc = false;
         if (rc == B200ATTN_OK) done = true;
         else if (rc != -1) return rc;
+        if (!done && sw_supported(*c, *a)) {
+            rc = run_sw(*c, a, 1, rd, base, st);
+            if (rc == B200ATTN_OK) done = true;
+            else if (rc != -1) return rc;
+        }
     }
     if (!done) {
         rc = (a->dtype == B200ATTN_F32) ? run_splitd<float>(*c, *a, rd, base, st)
@@ -651,6 +742,37 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
         if (rc) return rc;
     }
     return check_kernel_errors(*c, st, !(a->flags & B200ATTN_FLAG_ASYNC));
+}
+
+// How many of the `n` entries from `a` on go out in one launch of the streamed split-head_d kernel: asynchronous fp32 entries
+// of one form on one stream, none of which touches another's output (entries are independent by contract, but an entry
+// that reads an earlier one's output has always been ordered after it), with at most a CTA per SM in all.  1: not a group.
+static int batch_group(const b200attn_args *a, int n) {
+    int rd, rd1; float base, base1;
+    DeviceCtx *c;
+    if (n < 2 || a->struct_size != sizeof *a || a->dtype != B200ATTN_F32 || !(a->flags & B200ATTN_FLAG_ASYNC) ||
+        (a->flags & (B200ATTN_FLAG_FORCE_GENERIC | B200ATTN_FLAG_FORCE_TWO_PASS)))
+        return 1;
+    if (validate(a, &rd, &base) || get_ctx(&c) || !sw_supported(*c, *a)) return 1;
+    const long long BH = (long long)a->batch_sz * a->num_heads;
+    long long most = c->sm_count / BH;
+    if (most > SW_MAXP) most = SW_MAXP;
+    const size_t qb = (size_t)BH * a->len_q * a->head_d * 4, kb = (size_t)BH * a->len_k * a->head_d * 4;
+    auto meet = [](const void *x, size_t nx, const void *y, size_t ny) { return (uintptr_t)x < (uintptr_t)y + ny && (uintptr_t)y < (uintptr_t)x + nx; };
+    int g = 1;
+    for (; g < n && g < most; ++g) {
+        const b200attn_args &b = a[g];
+        if (b.struct_size != sizeof b || b.dtype != a->dtype || b.flags != a->flags || (b.flags & B200ATTN_FLAG_NO_OVERLAP) || b.stream != a->stream || b.pe != a->pe ||
+            (long long)b.batch_sz * b.num_heads != BH || b.len_q != a->len_q || b.len_k != a->len_k || b.head_d != a->head_d || b.cos_cache != a->cos_cache)
+            break;
+        if (validate(&b, &rd1, &base1) || rd1 != rd || base1 != base || !sw_supported(*c, b)) break;
+        bool apart = true;
+        for (int i = 0; i < g && apart; ++i)
+            apart = !meet(a[i].out, qb, b.out, qb) && !meet(a[i].out, qb, b.Q, qb) && !meet(a[i].out, qb, b.K, kb) && !meet(a[i].out, qb, b.V, kb) &&
+                    !meet(b.out, qb, a[i].Q, qb) && !meet(b.out, qb, a[i].K, kb) && !meet(b.out, qb, a[i].V, kb);
+        if (!apart) break;
+    }
+    return g;
 }
 
 static int ensure_stage(DeviceCtx &c, int i, size_t bytes) {
@@ -769,6 +891,12 @@ int b200attn_debug_tc_prof(unsigned long long *out32, int reset) {
 int b200attn_forward_many(const b200attn_args *args, int n) {
     if (args == nullptr || n < 0) return fail(B200ATTN_ERR_INVALID_ARG, "b200attn_forward_many: NULL args or negative n");
     for (int i = 0; i < n; ++i) {
+        const int g = batch_group(args + i, n - i);
+        if (g > 1) {
+            int rc = forward_device(&args[i], false, false, g);
+            if (rc == B200ATTN_OK) { i += g - 1; continue; }
+            if (rc != -1) return rc;
+        }
         // the entries are independent problems by contract: entry i may overlap the tail of entry i - 1
         const bool beside_prev = i > 0 && !(args[i].flags & B200ATTN_FLAG_NO_OVERLAP);
         const bool beside_next = i + 1 < n && !(args[i + 1].flags & B200ATTN_FLAG_NO_OVERLAP);
@@ -1021,6 +1149,7 @@ void b200attn_release_workspace(void) {
         for (int i = 0; i < 8; ++i) { if (c.stage[i]) cudaFree(c.stage[i]); c.stage[i] = nullptr; c.stage_bytes[i] = 0; }
         c.tc_tables.release();
         c.tcw.release();
+        c.sw_tables.release();
         c.prev_sdtc = false;
     }
     cudaSetDevice(prev);

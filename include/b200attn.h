@@ -158,7 +158,8 @@ int b200attn_forward_ex(const b200attn_args *args);
  * to back without a host synchronisation in between), with one difference: because no entry may read
  * what another entry of the same call writes, the library lets consecutive entries on one stream
  * overlap on the GPU (entry i starts loading its inputs while entry i-1 is finishing; an entry whose
- * Q, K or V overlaps the previous entry's `out` is simply not overlapped). */
+ * Q, K or V overlaps the previous entry's `out` is simply not overlapped).  Consecutive asynchronous fp32
+ * entries of one form (shape, encoding, flags, stream) whose tensors do not overlap may go out in one launch. */
 int b200attn_forward_many(const b200attn_args *args, int n);
 
 /* Same computation with HOST buffers (pageable or pinned): copies Q, K, V to device staging
@@ -182,8 +183,8 @@ void b200attn_shard_ranges(long long total_bh, int n_parts, long long *begin, lo
 const char *b200attn_last_error(void);
 
 /* Name of the kernel path the last successful b200attn_forward_ex on this thread used:
- * "splitd_tc" (fp32, short sequences, tensor cores with error-compensated tf32), "splitd_fused" and
- * "splitd_two_pass" (CUDA cores), "tc_wide" (bf16 on the tensor cores: score kernel, then P V kernel),
+ * "splitd_tc" (fp32, short sequences, tensor cores with error-compensated tf32), "splitd_stream" (short
+ * sequences of any type on the tensor cores, streamed slices), "splitd_fused" and "splitd_two_pass" (CUDA cores), "tc_wide" (bf16 on the tensor cores: score kernel, then P V kernel),
  * "tc_fused" (bf16 / fp16, head_d up to 256 in steps of 8, more than 64 queries: one kernel, scores in tensor
  * memory; an encoding is applied to copies of Q and K first), "tc_bf16" (bf16 on the tensor cores, one-kernel
  * cluster pipeline) or "tc_decode" (bf16, up to 64 queries against a long K/V: key splits on the tensor cores

@@ -1,0 +1,120 @@
+"""The streamed split-head_d kernel (csrc/splitd_stream.cuh) against the oracle: slices around its units (atoms of 32 columns, groups and
+blocks of four), 16-bit tensors, encodings, several problems in one launch."""
+import numpy as np
+import pytest
+import torch
+
+import oracle_lib as ol
+from gpu_util import bf16_from_dev, bf16_problem, bf16_to_dev, to_dev
+
+pytestmark = pytest.mark.gpu
+MAX_ABS = 5e-6   # fp32, uniform inputs: the library errs by 1e-7 of outputs below 1, the fp32 oracle by ~1e-6
+
+def attention64(Q, K, V, pe=ol.PE_NONE):
+    """The oracle's mathematics in 64 bits, on its own fp32 tables where the encoding is the additive one: a row's scores are then
+    near head_d / 2 before the scaling, and the fp32 oracle's sum of head_d terms errs by more than the bounds here."""
+    Q, K, V = (x.astype(np.float64) for x in (Q, K, V))
+    if pe == ol.PE_SINUSOIDAL:
+        D = Q.shape[-1]
+        s, c = ol.sinusoidal_tables(max(Q.shape[2], K.shape[2]), D)
+        tab = np.where(np.arange(D) % 2 == 0, s, c)   # a pair's columns both hold its value
+        Q, K = Q + tab[:Q.shape[2]], K + tab[:K.shape[2]]
+    S = Q @ K.swapaxes(-1, -2) / np.sqrt(Q.shape[-1])
+    P = np.exp(S - S.max(-1, keepdims=True))
+    return P / P.sum(-1, keepdims=True) @ V
+
+
+def want_of(Q, K, V, pe):
+    return attention64(Q, K, V, pe) if pe == ol.PE_SINUSOIDAL else ol.attention(Q, K, V, pe=pe)
+
+
+def bound(pe, D):
+    """Largest difference, for values up to 1 or so.  The host's and the device's fp32 frequencies differ by an ulp or two: up to
+    63 * 2^-23 of an angle at position 63, which enters a score of the additive encoding with the weights of head_d / 2 pairs of
+    magnitude 1 (over sqrt(head_d)), one of the rotation with those of products of inputs."""
+    return {ol.PE_NONE: MAX_ABS, ol.PE_SINUSOIDAL: 63 * 2.0 ** -23 * D ** 0.5}.get(pe, 5e-5)
+
+
+# heads x head_d such that a CTA has 9 to 33 atoms (one slice per head up to a few), odd lengths, a partial last atom and block
+WIDE = [(1, 148, 16, 16, 300), (1, 100, 33, 17, 1000), (1, 74, 64, 64, 1056), (1, 37, 1, 64, 2052), (1, 140, 50, 49, 128), (1, 20, 64, 48, 4096), (1, 148, 64, 1, 32)]
+
+
+@pytest.mark.parametrize("shape", WIDE, ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("pe", [ol.PE_NONE, ol.PE_ROPE_INTERLEAVED, ol.PE_SINUSOIDAL])
+def test_fp32(pkg, cuda, shape, pe):
+    B, H, Lq, Lk, D = shape
+    Q, K, V = ol.make_qkv(B, H, Lq, Lk, D, 90, "uniform")
+    want = want_of(Q, K, V, pe)
+    q, k, v = (to_dev(x, cuda) for x in (Q, K, V))
+    for rep in range(2):
+        got = pkg.forward(q, k, v, pe=pe).cpu().numpy()
+        # (a slice of up to 256 columns without an encoding fits the kernel that keeps V in shared memory)
+        assert pkg.last_path() in (("splitd_stream", "splitd_tc") if pe == ol.PE_NONE else ("splitd_stream",))
+        res = ol.compare(got, want)
+        assert res["max_abs"] <= bound(pe, D), (shape, pe, res)
+
+
+@pytest.mark.parametrize("D,rd", [(36, 0), (64, 6), (200, 34)])
+@pytest.mark.parametrize("pe", [ol.PE_ROPE_INTERLEAVED, ol.PE_ROPE_Q_ONLY])
+def test_partial_rotary(pkg, cuda, D, rd, pe):
+    Q, K, V = ol.make_qkv(2, 3, 30, 61, D, 91, "uniform")
+    got = pkg.forward(to_dev(Q, cuda), to_dev(K, cuda), to_dev(V, cuda), pe=pe, rotary_dim=rd, rope_base=500.0).cpu().numpy()
+    assert pkg.last_path() == "splitd_stream"
+    res = ol.compare(got, ol.attention(Q, K, V, pe=pe, rotary_dim=rd or None, base=500.0))
+    assert res["ok"] and res["max_abs"] <= 5e-5, res
+
+
+@pytest.mark.parametrize("shape", [(1, 4, 64, 64, 512), (1, 148, 17, 33, 200), (1, 9, 64, 31, 4096), (1, 60, 5, 64, 1032)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("pe", [ol.PE_NONE, ol.PE_ROPE_INTERLEAVED, ol.PE_SINUSOIDAL])
+@pytest.mark.parametrize("f16", [False, True])
+def test_16_bit(pkg, cuda, shape, pe, f16):
+    B, H, Lq, Lk, D = shape
+    if f16:
+        T = [x.astype(np.float16) for x in ol.make_qkv(B, H, Lq, Lk, D, 92, "normal")]
+        up = [x.astype(np.float32) for x in T]
+        got = pkg.forward(*(to_dev(x, cuda) for x in T), pe=pe).float().cpu().numpy()
+    else:
+        bits, up = bf16_problem(B, H, Lq, Lk, D, 92)
+        got = bf16_from_dev(pkg.forward(*(bf16_to_dev(b, cuda) for b in bits), pe=pe))
+    assert pkg.last_path() == "splitd_stream"
+    want = want_of(*up, pe)
+    # everything up to the output is fp32: half a unit in the last place of the output's format, and what fp32 differs by
+    err = np.abs(got - want)
+    assert (err <= np.abs(want) * (2.0 ** -11 if f16 else 2.0 ** -8) + 4 * max(bound(pe, D), 5e-5)).all(), err.max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_non_finite_values_as_on_the_cuda_cores(pkg, cuda, dtype, which, value):
+    T = [to_dev(x, cuda).to(dtype) for x in ol.make_qkv(1, 3, 50, 50, 304, 93, "uniform")]
+    T[which][0, 1, 7, 5] = value
+    got = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED)
+    assert pkg.last_path() == "splitd_stream"
+    want = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED, flags=pkg.FLAG_FORCE_GENERIC)
+    assert pkg.last_path() == "splitd_fused"
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+
+
+@pytest.mark.parametrize("pe", [ol.PE_NONE, ol.PE_SINUSOIDAL])
+@pytest.mark.parametrize("H,Lq,Lk,D,n", [(4, 64, 64, 512, 5), (1, 16, 64, 64, 17), (30, 33, 20, 1000, 6), (148, 8, 8, 64, 2)])
+def test_one_launch_for_several_problems(pkg, cuda, pe, H, Lq, Lk, D, n):
+    """Equal entries of a batch share launches; an entry that reads an earlier one's output still sees it."""
+    probs, args = [], []
+    for i in range(n):
+        Q, K, V = ol.make_qkv(1, H, Lq, Lk, D, 100 + i, "uniform")
+        q, k, v = (to_dev(x, cuda) for x in (Q, K, V))
+        probs.append((Q, K, V, q, k, v, torch.full_like(q, float("nan"))))
+        args.append(pkg.args_for(q, k, v, probs[-1][-1], pe=pe, flags=pkg.FLAG_ASYNC))
+    o2 = torch.full_like(probs[0][3], float("nan"))
+    args.append(pkg.args_for(probs[1][-1], probs[0][4], probs[0][5], o2, pe=pe, flags=pkg.FLAG_ASYNC))
+    n0 = pkg.launch_count()
+    for _ in range(2):
+        pkg.forward_many(args)
+    torch.cuda.synchronize()
+    if n * H <= 16:
+        assert pkg.launch_count() - n0 < 2 * len(args)
+    for Q, K, V, _, _, _, o in probs:
+        res = ol.compare(o.cpu().numpy(), ol.attention(Q, K, V, pe=pe))
+        assert res["ok"] and res["max_abs"] <= 5e-5, res
+    assert ol.compare(o2.cpu().numpy(), ol.attention(probs[1][-1].cpu().numpy(), probs[0][1], probs[0][2], pe=pe))["ok"]
