@@ -25,6 +25,7 @@
 #include "tc_wide.cuh"
 #include "dec.cuh"
 #include "tc_fa.cuh"
+#include "tc_f32.cuh"
 
 namespace b200attn {
 
@@ -127,6 +128,7 @@ struct DeviceCtx {
     TmapCache tmaps;
     TcTables tc_tables;            // positional-encoding tables of the tensor-core path
     TcwScratch tcw;                // scratch of the wide-head tensor-core path
+    F32Scratch f32;                // scratch of the fp32 path for longer sequences
 };
 static DeviceCtx g_ctx[kMaxDevices];
 
@@ -724,6 +726,11 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
             else if (rc != -1) return fail(rc, "%s", tc_bf16_error());
         }
     }
+    if (!done && !(a->flags & (B200ATTN_FLAG_FORCE_GENERIC | B200ATTN_FLAG_FORCE_TWO_PASS)) && f32tc_supported(*a)) {
+        rc = f32tc_run(*a, rd, base, c->f32, c->err_dev, c->err_host_dev, c->sm_count, current_spin_limit(), (size_t)g_score_scratch_mb.load() << 20, st, &g_launches);
+        if (rc == B200ATTN_OK) { t_last_path = "tc_f32"; done = true; }
+        else if (rc != -1) return fail(rc, "%s", tc_bf16_error());
+    }
     if (!done && !(a->flags & (B200ATTN_FLAG_FORCE_GENERIC | B200ATTN_FLAG_FORCE_TWO_PASS))) {
         c->prev_sdtc = chain;
         rc = run_sdtc(*c, *a, st, independent_of_prev, batched);
@@ -1149,6 +1156,7 @@ void b200attn_release_workspace(void) {
         for (int i = 0; i < 8; ++i) { if (c.stage[i]) cudaFree(c.stage[i]); c.stage[i] = nullptr; c.stage_bytes[i] = 0; }
         c.tc_tables.release();
         c.tcw.release();
+        c.f32.release();
         c.sw_tables.release();
         c.prev_sdtc = false;
     }

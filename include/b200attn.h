@@ -184,7 +184,8 @@ const char *b200attn_last_error(void);
 
 /* Name of the kernel path the last successful b200attn_forward_ex on this thread used:
  * "splitd_tc" (fp32, short sequences, tensor cores with error-compensated tf32), "splitd_stream" (short
- * sequences of any type on the tensor cores, streamed slices), "splitd_fused" and "splitd_two_pass" (CUDA cores), "tc_wide" (bf16 on the tensor cores: score kernel, then P V kernel),
+ * sequences of any type on the tensor cores, streamed slices), "tc_f32" (fp32, longer sequences, head_d up to 512:
+ * three kernels on bf16 pieces of the operands), "splitd_fused" and "splitd_two_pass" (CUDA cores), "tc_wide" (bf16 on the tensor cores: score kernel, then P V kernel),
  * "tc_fused" (bf16 / fp16, head_d up to 256 in steps of 8, more than 64 queries: one kernel, scores in tensor
  * memory; an encoding is applied to copies of Q and K first), "tc_bf16" (bf16 on the tensor cores, one-kernel
  * cluster pipeline) or "tc_decode" (bf16, up to 64 queries against a long K/V: key splits on the tensor cores
@@ -214,7 +215,7 @@ int b200attn_rope_k(const void *X, void *X_rot, int batch_sz, int num_heads, int
 
 /* Process-wide settings (they apply to calls made after the change). */
 enum b200attn_option {
-    B200ATTN_OPT_SCORE_SCRATCH_MB = 1, /* bf16 two-kernel path: cap, in MiB, of the score scratch of one pass over the heads (default 2048) */
+    B200ATTN_OPT_SCORE_SCRATCH_MB = 1, /* bf16 two-kernel path and tc_f32: cap, in MiB, of the score scratch of one pass over the heads (default 2048) */
     B200ATTN_OPT_SPIN_LIMIT = 2        /* polls after which a wait inside a kernel gives up and reports B200ATTN_ERR_KERNEL (default 2^21) */
 };
 int b200attn_set_option(int option, long long value);
