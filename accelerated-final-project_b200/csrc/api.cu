@@ -476,6 +476,7 @@ static int run_sdtc(DeviceCtx &c, const b200attn_args &a, cudaStream_t st, bool 
     p.err = c.err_dev; p.err_sys = c.err_host_dev;
     p.spin_limit = current_spin_limit();
     p.wait_extra = g_test_wait_extra.load();
+    p.wait_first = overlap ? 0 : 1;
 #ifdef B200ATTN_DEVTOOLS
     p.dbg = g_sdtc_dbg;
     p.stamps = g_sdtc_stamps;
@@ -491,7 +492,7 @@ static int run_sdtc(DeviceCtx &c, const b200attn_args &a, cudaStream_t st, bool 
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     CU_TRY(cudaLaunchKernelEx(&cfg, sdtc_kernel, tmQ, tmK, tmV, p));

@@ -185,6 +185,8 @@ dec_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t tmem = tmem_slot;
     const uint32_t tmem_s = tmem, tmem_o = tmem + 256;   // S buffers at columns 0 / 128, output buffers at 256 / 384
     bool failed = false;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const bool skip = (*reinterpret_cast<volatile unsigned *>(p.err) != 0);
 
     if (skip) {
@@ -457,6 +459,8 @@ dec_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     const uint32_t tmem = tmem_slot;
     const uint32_t tmem_s = tmem, tmem_o = tmem + 128;   // St buffers at columns 0 / 64, Ot buffers at 128 / 192
     bool failed = false;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const bool skip = (*reinterpret_cast<volatile unsigned *>(p.err) != 0);
 
     if (skip) {
@@ -660,6 +664,8 @@ dec_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
 
 // out[bh][i][:] from the splits' (max, sum, O): grid (Lq, BH), one thread per output column pair.
 __global__ void dec_combine_kernel(const DecParams p) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int i = blockIdx.x;
     const long long bh = blockIdx.y;
     const float *ml = p.part_ml + (bh * p.nsplit * DC_MQ + i) * 2;
@@ -778,15 +784,15 @@ inline int dec_run(const b200attn_args &a, int rd, float base, TcwScratch &sc, T
     const dim3 grid((unsigned)p.nsplit, (unsigned)BH);
     const size_t smem = dec_smem_bytes(nch);
     // up to 32 queries: the transposed kernel (keys along the tensor-memory lanes); more: a row per query
-    if (Lq <= 16) { if (nch == 1) dec_t_kernel<1, 16><<<grid, DC_THREADS, smem, st>>>(tmQ, tmK, tmV, p); else dec_t_kernel<2, 16><<<grid, DC_THREADS, smem, st>>>(tmQ, tmK, tmV, p); }
-    else if (Lq <= 32) { if (nch == 1) dec_t_kernel<1, 32><<<grid, DC_THREADS, smem, st>>>(tmQ, tmK, tmV, p); else dec_t_kernel<2, 32><<<grid, DC_THREADS, smem, st>>>(tmQ, tmK, tmV, p); }
-    else if (nch == 1) dec_split_kernel<1><<<grid, DC_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
-    else dec_split_kernel<2><<<grid, DC_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
+    if (Lq <= 16) { if (nch == 1) launch_dependent(dec_t_kernel<1, 16>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); else launch_dependent(dec_t_kernel<2, 16>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); }
+    else if (Lq <= 32) { if (nch == 1) launch_dependent(dec_t_kernel<1, 32>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); else launch_dependent(dec_t_kernel<2, 32>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); }
+    else if (nch == 1) launch_dependent(dec_split_kernel<1>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p);
+    else launch_dependent(dec_split_kernel<2>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "dec_split_kernel launch failed: %s", cudaGetErrorString(e)); return B200ATTN_ERR_CUDA; }
     launches->fetch_add(1);
     if (p.nsplit > 1) {
-        dec_combine_kernel<<<dim3((unsigned)Lq, (unsigned)BH), 64, 0, st>>>(p);
+        launch_dependent(dec_combine_kernel, dim3((unsigned)Lq, (unsigned)BH), 64, 0, 1, st, p);
         e = cudaGetLastError();
         if (e != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "dec_combine_kernel launch failed: %s", cudaGetErrorString(e)); return B200ATTN_ERR_CUDA; }
         launches->fetch_add(1);

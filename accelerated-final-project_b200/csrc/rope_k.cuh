@@ -14,7 +14,7 @@
 // attention call of 8 x 12 heads, 1000 x 1000, head_d 64 with its two encoding launches: 166 us; now 72 us).
 #pragma once
 
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace b200attn {
 
@@ -92,6 +92,8 @@ __device__ __forceinline__ void rope_angle(const RopeKParams &p, int pos, int pa
 // (D - rd)/N copy vectors.  gridDim.y shares the slices.
 template <typename T>
 __global__ void __launch_bounds__(256) rope_k_vec_kernel(const RopeKParams p) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     constexpr int N = RopeVec<T>::N;
     const T *X = reinterpret_cast<const T *>(blockIdx.z ? p.X2 : p.X);
     T *Y = reinterpret_cast<T *>(blockIdx.z ? p.Y2 : p.Y);
@@ -166,6 +168,8 @@ __global__ void __launch_bounds__(256) rope_k_vec_kernel(const RopeKParams p) {
 // Any shape and alignment: a thread owns one pair (or one copied column) of one row.
 template <typename T>
 __global__ void __launch_bounds__(256) rope_k_scalar_kernel(const RopeKParams p) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const T *X = reinterpret_cast<const T *>(blockIdx.z ? p.X2 : p.X);
     T *Y = reinterpret_cast<T *>(blockIdx.z ? p.Y2 : p.Y);
     const int L = blockIdx.z ? p.L2 : p.L;
@@ -211,9 +215,7 @@ inline cudaError_t launch_rope_k(const RopeKParams &p, int sm_count, cudaStream_
     if (shares > 65535) shares = 65535;
     if (shares < 1) shares = 1;
     const dim3 grid((unsigned)blocks, (unsigned)shares, two ? 2 : 1);
-    if (vec) rope_k_vec_kernel<T><<<grid, 256, 0, st>>>(p);
-    else rope_k_scalar_kernel<T><<<grid, 256, 0, st>>>(p);
-    return cudaGetLastError();
+    return vec ? launch_dependent(rope_k_vec_kernel<T>, grid, 256, 0, 1, st, p) : launch_dependent(rope_k_scalar_kernel<T>, grid, 256, 0, 1, st, p);
 }
 
 }  // namespace b200attn

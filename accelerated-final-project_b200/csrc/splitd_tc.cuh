@@ -80,6 +80,7 @@ struct SdtcParams {
     unsigned *err, *err_sys;
     unsigned spin_limit;
     unsigned wait_extra;     // 0; a test makes the head wait for arrivals that never come
+    int wait_first;          // the call starts after what precedes it in the stream: wait for that before touching global memory
 #ifdef B200ATTN_DEVTOOLS
     float *dbg;              // bring-up dump of CTA (0, 0): see the ST_DBG sites
     unsigned long long *stamps;   // [CTAs][32] globaltimer at the ST_STAMP sites
@@ -245,6 +246,7 @@ sdtc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         mbar_init(&bars.buf_ok, 1);
         s_fail = 0u;
         mbar_fence_init();
+        if (p.wait_first) grid_dependency_wait();
         for (int c = 0; c < nat && c < nr; ++c) load_atom(c, c);
         mbar_expect_tx(&bars.v_full, (uint32_t)nat * (uint32_t)Lk * 128u);
         if (p.v_own) load_v();
@@ -256,7 +258,8 @@ sdtc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     const uint32_t tmem = tmem_slot;
     bool failed = false;
     if (threadIdx.x == 0) ST_STAMP(1);
-    // a following call that was declared independent of this one may start its loads now
+    // a following call that was declared independent of this one may start its loads now (but not before what both follow is complete)
+    if (p.wait_first) grid_dependency_wait();
     grid_launch_dependents();
 
     if (warp == 0) {

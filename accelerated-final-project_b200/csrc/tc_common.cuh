@@ -238,7 +238,7 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 // Launches a kernel as the programmatic dependent of whatever precedes it in the stream: it may be set up while that still runs,
 // and must call grid_dependency_wait before it touches global memory.  `cluster`: CTAs per cluster along x.
 template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, A &&...args) {
+inline cudaError_t launch_kernel(bool dependent, void (*kern)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, A &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
@@ -246,13 +246,22 @@ inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, int threads, 
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = dependent ? 1 : 0;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = (unsigned)cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, A &&...args) {
+    return launch_kernel(true, kern, grid, threads, smem, cluster, st, std::forward<A>(args)...);
+}
+// Whether the launches of a long-running call are worth making dependent.  A dependent launch saves 2 to 5 us (22 heads, 591 x 591,
+// head_d 512, bf16, two launches: 40.5 -> 35.4 us; 10 heads, 619 x 619, head_d 1024, sinusoidal, three: 66.7 -> 64.2 us), but the
+// CTAs that come to wait on an SM while their neighbours still compute cost a power-capped call more than that (128 heads, 2048 x
+// 2048, head_d 1024: 2550 -> 2592 us; 512 heads, 4096 x 4096, head_d 512: 20.15 -> 20.34 ms; 28 heads, 2866 x 2866: 1124 -> 1129 us).
+inline bool worth_dependent(long long BH, long long Lq, long long Lk, long long D) { return 4.0 * BH * Lq * Lk * D <= 2e11; }
 
 // ---- TMA tiled store shared -> global (bulk async-group completion) ---------------------------------
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *tmap, const void *smem_src, int x, int y) {

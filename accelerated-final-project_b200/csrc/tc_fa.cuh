@@ -183,6 +183,8 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
     tc_fence_after();
     const uint32_t tmem = tmem_slot;        // S_t: columns [128 t, 128 t + 128); O_t: [256 + 128 t, ...)
     bool failed = false;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const bool skip = (*reinterpret_cast<volatile unsigned *>(p.err) != 0);   // an earlier kernel of the call failed
 
     // the softmax threads hold a whole score row: they take over registers that the loading and issuing warps do not need
@@ -475,6 +477,8 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     tc_fence_after();
     const uint32_t tmem = tmem_slot;        // score buffer b: columns [128 b, 128 b + 128); O: [256, 512)
     bool failed = false;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const bool skip = (*reinterpret_cast<volatile unsigned *>(p.err) != 0);
 
     if (skip) {
@@ -779,8 +783,8 @@ inline int fa_run(const b200attn_args &a, unsigned *err_dev, unsigned *err_sys, 
         p.err = err_dev; p.err_sys = err_sys; p.spin_limit = spin_limit;
         const unsigned grid = (unsigned)(p.n_units < sm_count ? p.n_units : sm_count);
         const size_t smem = (size_t)(2 + nst) * FB_STAGE + 1024;
-        if (p.f16) fa256_kernel<true><<<grid, FB_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
-        else fa256_kernel<false><<<grid, FB_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
+        if (p.f16) launch_kernel(worth_dependent(BH, Lq, Lk, D), fa256_kernel<true>, dim3(grid), FB_THREADS, smem, 1, st, tmQ, tmK, tmV, p);
+        else launch_kernel(worth_dependent(BH, Lq, Lk, D), fa256_kernel<false>, dim3(grid), FB_THREADS, smem, 1, st, tmQ, tmK, tmV, p);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "fa256_kernel launch failed: %s", cudaGetErrorString(e)); return B200ATTN_ERR_CUDA; }
         launches->fetch_add(1);
@@ -807,8 +811,8 @@ inline int fa_run(const b200attn_args &a, unsigned *err_dev, unsigned *err_sys, 
     p.err = err_dev; p.err_sys = err_sys; p.spin_limit = spin_limit;
     const unsigned grid = (unsigned)(p.n_units < sm_count ? p.n_units : sm_count);
     const size_t smem = 2 * tb + 2 * (size_t)FA_P_BYTES + (size_t)nst * tb + 1024;
-    if (p.f16) fa_kernel<true><<<grid, FA_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
-    else fa_kernel<false><<<grid, FA_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
+    if (p.f16) launch_kernel(worth_dependent(BH, Lq, Lk, D), fa_kernel<true>, dim3(grid), FA_THREADS, smem, 1, st, tmQ, tmK, tmV, p);
+    else launch_kernel(worth_dependent(BH, Lq, Lk, D), fa_kernel<false>, dim3(grid), FA_THREADS, smem, 1, st, tmQ, tmK, tmV, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "fa_kernel launch failed: %s", cudaGetErrorString(e)); return B200ATTN_ERR_CUDA; }
     launches->fetch_add(1);

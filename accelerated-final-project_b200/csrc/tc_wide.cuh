@@ -226,6 +226,8 @@ tcw_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool failed = false;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const bool skip = (*reinterpret_cast<volatile unsigned *>(p.err) != 0);   // an earlier kernel of the call failed
 
     if (skip) {
@@ -526,6 +528,8 @@ tcw_scores256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool failed = false;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const bool skip = (*reinterpret_cast<volatile unsigned *>(p.err) != 0);
 
     if (skip) {
@@ -674,6 +678,8 @@ tcw_pv_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ C
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool failed = false;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const bool skip = (*reinterpret_cast<volatile unsigned *>(p.err) != 0);
 
     if (skip) {
@@ -1124,8 +1130,8 @@ inline int tcw_run(const b200attn_args &a, int rd, float base, TcwScratch &sc, T
             sp.mode = mode; sp.tph = tph; sp.n_tiles = nh * tph;
             const unsigned grid = (unsigned)(sp.n_tiles < sm_count ? sp.n_tiles : sm_count);
             tcw_timer().begin(mode == 1 ? 0 : 1, st);
-            if (big) tcw_scores256_kernel<<<grid, T2_THREADS, (size_t)T2_NST * T2_STAGE + 1024, st>>>(tmQ, tmK, sp);
-            else tcw_scores_kernel<<<grid, TW_THREADS, smem_s, st>>>(tmQ, tmK, sp);
+            if (big) launch_kernel(worth_dependent(BH, Lq, Lk, D), tcw_scores256_kernel, dim3(grid), T2_THREADS, (size_t)T2_NST * T2_STAGE + 1024, 1, st, tmQ, tmK, sp);
+            else launch_kernel(worth_dependent(BH, Lq, Lk, D), tcw_scores_kernel, dim3(grid), TW_THREADS, smem_s, 1, st, tmQ, tmK, sp);
             tcw_timer().end(st);
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "score kernel launch failed: %s", cudaGetErrorString(e)); return B200ATTN_ERR_CUDA; }
@@ -1153,7 +1159,7 @@ inline int tcw_run(const b200attn_args &a, int rd, float base, TcwScratch &sc, T
         tcw_timer().begin(2, st);
         {
             const unsigned grid = (unsigned)(pp.n_units < sm_count ? pp.n_units : sm_count);
-            tcw_pv_kernel<<<grid, TP_THREADS, smem_p, st>>>(tmV, tmS, pp);
+            launch_kernel(worth_dependent(BH, Lq, Lk, D), tcw_pv_kernel, dim3(grid), TP_THREADS, smem_p, 1, st, tmV, tmS, pp);
         }
         tcw_timer().end(st);
         cudaError_t e = cudaGetLastError();
