@@ -36,6 +36,9 @@ class Args(C.Structure):
     ]
 
 
+_ARGS_SIZE = C.sizeof(Args)
+
+
 class B200AttnError(RuntimeError):
     def __init__(self, status, message):
         super().__init__(f"b200attn status {status}: {message}")
@@ -103,9 +106,22 @@ def make_args(Q, K, V, out, B, H, Lq, Lk, D, dtype, pe=PE_NONE, rotary_dim=0, ro
                 cos_cache, sin_cache, stream, flags)
 
 
+_torch = _DTYPES = None
+
+
+def _with_torch():
+    """torch, imported on first use (the binding itself does not need it)."""
+    global _torch, _DTYPES
+    if _torch is None:
+        import torch
+        _DTYPES = {torch.float32: F32, torch.bfloat16: BF16, torch.float16: F16}
+        _torch = torch
+    return _torch
+
+
 def dtype_of(t):
-    import torch
-    return {torch.float32: F32, torch.bfloat16: BF16, torch.float16: F16}[t.dtype]
+    _with_torch()
+    return _DTYPES[t.dtype]
 
 
 def check(status):
@@ -117,20 +133,28 @@ def forward(Q, K, V, out=None, pe=PE_NONE, rotary_dim=0, rope_base=0.0, cos_cach
             stream=None, flags=0):
     """Attention forward on torch CUDA tensors Q [B,H,Lq,D], K/V [B,H,Lk,D] (float32 or bfloat16,
     contiguous) through b200attn_forward_ex.  Returns `out`."""
-    import torch
+    # (a short call is bound by this function: 10.5 us of interpreter per call, against 10 us of GPU, with a torch.cuda.device block
+    # around every call, a Stream object made to read its handle and the imports and tables set up again; 4 x 64 x 64, head_d 512)
+    torch = _torch or _with_torch()
     assert Q.is_cuda and K.is_cuda and V.is_cuda and Q.is_contiguous() and K.is_contiguous() and V.is_contiguous()
     B, H, Lq, D = Q.shape
-    Lk = K.shape[2]
-    dtype = dtype_of(Q)
+    dtype = _DTYPES[Q.dtype]
     if out is None:
         out = torch.empty_like(Q)
+    dev = Q.get_device()
     if stream is None:
-        stream = torch.cuda.current_stream(Q.device).cuda_stream
-    a = make_args(Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), B, H, Lq, Lk, D, dtype, pe, rotary_dim,
-                  rope_base, cos_cache.data_ptr() if cos_cache is not None else None,
-                  sin_cache.data_ptr() if sin_cache is not None else None, stream, flags)
-    with torch.cuda.device(Q.device):
-        check(lib().b200attn_forward_ex(C.byref(a)))
+        stream = torch._C._cuda_getCurrentRawStream(dev)
+    a = Args(_ARGS_SIZE, Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), B, H, Lq, K.shape[2], D, dtype, pe, rotary_dim,
+             rope_base, cos_cache.data_ptr() if cos_cache is not None else None,
+             sin_cache.data_ptr() if sin_cache is not None else None, stream, flags)
+    fn = (_lib or lib()).b200attn_forward_ex
+    if dev == torch.cuda.current_device():
+        status = fn(C.byref(a))
+    else:
+        with torch.cuda.device(dev):
+            status = fn(C.byref(a))
+    if status != OK:
+        check(status)
     return out
 
 
