@@ -37,7 +37,9 @@ constexpr int DC_PBUF = 2 * DC_QSLAB;   // P [64 x 128 keys]: two atoms of 64 ke
 struct DecParams {
     long long BH;
     int Lq, Lk, D, nch;        // nch = D / 64
-    int nsplit, cps;           // key splits per head, chunks per split
+    int nsplit, cps;           // dec_split_kernel: key splits per head, chunks per split; both kernels: partial outputs kept per head
+    int chunks;                // chunks of 128 keys per head
+    int ctas;                  // dec_t_kernel: its grid; CTA i takes the chunks [i T / ctas, (i + 1) T / ctas) of the T = BH * chunks (0: dec_split_kernel)
     float scale_log2;          // log2(e) / sqrt(D)
     int table_kind;            // 0 none, 1 element-wise partner table (interleaved RoPE, sinusoidal), 2 rotate-half table
     int sinus, rotate_q, rotate_k;
@@ -49,6 +51,9 @@ struct DecParams {
     unsigned *err, *err_sys;
     unsigned spin_limit;
 };
+
+// the CTA of dec_t_kernel that takes chunk u
+__host__ __device__ inline int dec_cta_of(const DecParams &p, long long u) { return (int)(((u + 1) * p.ctas - 1) / (p.BH * p.chunks)); }
 
 struct DcBars {
     uint64_t q_full, q_ready;
@@ -401,6 +406,11 @@ dec_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // thread instead of 128.  The reference maximum of P is the RUNNING row maximum, the same for all
 // threads, so each thread rescales what it holds itself: its partial row sums (one per key lane, reduced
 // over the lanes once at the end of the split) and its row of the running Ot.
+//
+// The chunks of all heads are one sequence that the CTAs share out evenly, so a CTA runs through segments of up to a few
+// heads, Q double-buffered.  (Whole splits per CTA left SMs without work: 32 heads 128 of 148, 75 heads half of them.  bf16, 4
+// queries, 32768 keys, head_d 128, K rotated beforehand: 32
+// heads 108.9 -> 101.7 us; 4 queries, 8192 keys, 100 heads: 107 -> 83.8 us.)
 // ---------------------------------------------------------------------------------------------------
 template <int N> __device__ __forceinline__ void dec_tmem_ld(uint32_t taddr, uint32_t (&r)[N]);
 template <> __device__ __forceinline__ void dec_tmem_ld<32>(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
@@ -423,19 +433,26 @@ dec_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     __shared__ float wmax[2][4][NQ];   // chunk maxima of the four softmax warps, double-buffered by chunk parity
     __shared__ float wsum[4][NQ];
     __shared__ uint64_t mx_full[2], sum_full;   // the four warps have written wmax[i] / wsum (bounded waits, like every other)
+    __shared__ uint64_t q_full[2], q_ready[2], q_free[2];   // the Q buffers of alternating segments
     const uint32_t raw_addr = smem_u32(dc_smem_raw);
     unsigned char *smem = dc_smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int nch = NCH, D = 64 * NCH;
     const uint32_t lim = p.spin_limit;
-    const int split = blockIdx.x;
-    const long long bh = blockIdx.y;
-    const int total_chunks = (p.Lk + DC_NK - 1) / DC_NK;
-    const int c0 = split * p.cps, c1 = min(total_chunks, c0 + p.cps);
-    const int n = c1 - c0;
+    const long long T = p.BH * p.chunks, u0 = blockIdx.x * T / p.ctas, u1 = (blockIdx.x + 1) * T / p.ctas;
+    // segments: chunks [c0, c0 + n) of head bh, from chunk u of the sequence on
+    struct Seg { long long bh; int c0, n; };
+    auto segment = [&](long long u) {
+        Seg g;
+        g.bh = u / p.chunks;
+        g.c0 = (int)(u - g.bh * p.chunks);
+        g.n = (int)min((long long)(p.chunks - g.c0), u1 - u);
+        return g;
+    };
 
-    unsigned char *q_smem = smem;
-    unsigned char *k_smem = q_smem + (size_t)nch * DC_QSLAB;
+    constexpr int q_buf = nch * DC_QSLAB;
+    unsigned char *q_smem = smem;                                     // 2 buffers
+    unsigned char *k_smem = q_smem + (size_t)2 * q_buf;
     unsigned char *v_smem = k_smem + (size_t)2 * nch * DC_KSLAB;
     unsigned char *p_smem = v_smem + (size_t)2 * nch * DC_KSLAB;
     constexpr int kv_stage = nch * DC_KSLAB;
@@ -448,6 +465,7 @@ dec_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
             mbar_init(&bars.v_full[i], 1); mbar_init(&bars.v_free[i], 1);
             mbar_init(&bars.s_full[i], 1); mbar_init(&bars.p_full[i], 4); mbar_init(&bars.o_full[i], 1); mbar_init(&bars.o_free[i], 4);
         }
+        for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_ready[i], 4); mbar_init(&q_free[i], 1); }
         mbar_init(&mx_full[0], 4); mbar_init(&mx_full[1], 4); mbar_init(&sum_full, 4);
         mbar_fence_init();
         tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
@@ -467,43 +485,56 @@ dec_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
         // fall through to the common exit
     } else if (warp == 0) {
         if (lane == 0) {
-            mbar_expect_tx(&bars.q_full, (uint32_t)nch * (uint32_t)p.Lq * 128u);
-            for (int c = 0; c < nch; ++c) tma_load_2d(q_smem + (size_t)c * DC_QSLAB, &tmQ, c * 64, (int)(bh * p.Lq), &bars.q_full);
-            for (int t = 0; t < n; ++t) {
-                const int st = t & 1;
-                const int row0 = (int)(bh * p.Lk + (long long)(c0 + t) * DC_NK);
-                DC_FAIL_AT(0, !mbar_wait(&bars.k_free[st], ((t >> 1) & 1) ^ 1, lim));
-                mbar_expect_tx(&bars.k_full[st], (uint32_t)kv_stage);
-                tma_load_3d(k_smem + (size_t)st * kv_stage, &tmK, 0, row0, 0, &bars.k_full[st]);
-                DC_FAIL_AT(1, !mbar_wait(&bars.v_free[st], ((t >> 1) & 1) ^ 1, lim));
-                mbar_expect_tx(&bars.v_full[st], (uint32_t)kv_stage);
-                tma_load_3d(v_smem + (size_t)st * kv_stage, &tmV, 0, row0, 0, &bars.v_full[st]);
+            int k = 0, sg = 0;   // chunks, segments so far
+            for (long long u = u0; u < u1 && !failed; ++sg) {
+                const Seg g = segment(u);
+                const int qb = sg & 1;
+                DC_FAIL_AT(0, !mbar_wait(&q_free[qb], ((sg >> 1) & 1) ^ 1, lim));
+                mbar_expect_tx(&q_full[qb], (uint32_t)nch * (uint32_t)p.Lq * 128u);
+                for (int c = 0; c < nch; ++c) tma_load_2d(q_smem + qb * q_buf + (size_t)c * DC_QSLAB, &tmQ, c * 64, (int)(g.bh * p.Lq), &q_full[qb]);
+                for (int t = 0; t < g.n; ++t, ++k) {
+                    const int st = k & 1;
+                    const int row0 = (int)(g.bh * p.Lk + (long long)(g.c0 + t) * DC_NK);
+                    DC_FAIL_AT(0, !mbar_wait(&bars.k_free[st], ((k >> 1) & 1) ^ 1, lim));
+                    mbar_expect_tx(&bars.k_full[st], (uint32_t)kv_stage);
+                    tma_load_3d(k_smem + (size_t)st * kv_stage, &tmK, 0, row0, 0, &bars.k_full[st]);
+                    DC_FAIL_AT(1, !mbar_wait(&bars.v_free[st], ((k >> 1) & 1) ^ 1, lim));
+                    mbar_expect_tx(&bars.v_full[st], (uint32_t)kv_stage);
+                    tma_load_3d(v_smem + (size_t)st * kv_stage, &tmV, 0, row0, 0, &bars.v_full[st]);
+                }
+                u += g.n;
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t id_s = umma_idesc_16(DC_NK, NQ, 0, 0, p.f16), id_o = umma_idesc_16(D, NQ, 1, 0, p.f16);
-            auto issue_scores = [&](int t) -> bool {
-                const int st = t & 1;
-                if (!mbar_wait(p.rotate_k ? &bars.k_ready[st] : &bars.k_full[st], (t >> 1) & 1, lim)) return false;
+            const int total = (int)(u1 - u0);
+            int left = 0, sg = -1;   // score MMAs: chunks left in the segment, segment
+            auto issue_scores = [&](int k) -> bool {
+                const int st = k & 1;
+                if (left == 0) {
+                    left = segment(u0 + k).n;
+                    ++sg;
+                    if (!mbar_wait(p.rotate_q ? &q_ready[sg & 1] : &q_full[sg & 1], (sg >> 1) & 1, lim)) return false;
+                }
+                if (!mbar_wait(p.rotate_k ? &bars.k_ready[st] : &bars.k_full[st], (k >> 1) & 1, lim)) return false;
                 tc_fence_after();
                 for (int c = 0; c < nch; ++c) {
                     const uint64_t da = umma_desc_k_sw128(smem_u32(k_smem + (size_t)st * kv_stage + (size_t)c * DC_KSLAB));
-                    const uint64_t db = umma_desc_k_sw128(smem_u32(q_smem + (size_t)c * DC_QSLAB));
+                    const uint64_t db = umma_desc_k_sw128(smem_u32(q_smem + (sg & 1) * q_buf + (size_t)c * DC_QSLAB));
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_bf16(tmem_s + st * 64, da + 2 * k, db + 2 * k, id_s, (c | k) != 0);
+                    for (int kk = 0; kk < 4; ++kk) umma_bf16(tmem_s + st * 64, da + 2 * kk, db + 2 * kk, id_s, (c | kk) != 0);
                 }
                 umma_commit(&bars.k_free[st]);
                 umma_commit(&bars.s_full[st]);
+                if (--left == 0) umma_commit(&q_free[sg & 1]);
                 return true;
             };
             do {
-                DC_FAIL_AT(2, !mbar_wait(p.rotate_q ? &bars.q_ready : &bars.q_full, 0, lim));
-                tc_fence_after();
                 DC_FAIL_AT(3, !issue_scores(0));
-                for (int t = 0; t < n; ++t) {
+                for (int t = 0; t < total; ++t) {
                     const int st = t & 1;
-                    if (t + 1 < n) DC_FAIL_AT(4, !issue_scores(t + 1));
+                    if (t + 1 < total) DC_FAIL_AT(4, !issue_scores(t + 1));
                     DC_FAIL_AT(5, !mbar_wait(&bars.p_full[st], (t >> 1) & 1, lim));
                     DC_FAIL_AT(6, !mbar_wait(&bars.v_full[st], (t >> 1) & 1, lim));
                     DC_FAIL_AT(7, !mbar_wait(&bars.o_free[st], ((t >> 1) & 1) ^ 1, lim));
@@ -527,131 +558,145 @@ dec_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
         const int drow = (D == 128) ? j : 16 * qd + lane;
         const bool d_active = (D == 128) || lane < 16;
         float m_run[NQ], l_part[NQ], o_run[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) { m_run[q] = -INFINITY; l_part[q] = 0.0f; o_run[q] = 0.0f; }
         uint32_t r[NQ];
-        for (int t = 0; t < n && !failed; ++t) {
-            const int st = t & 1;
-            const bool valid = (c0 + t) * DC_NK + j < p.Lk;
-            DC_FAIL_AT(8, !mbar_wait(&bars.s_full[st], (t >> 1) & 1, lim));
-            tc_fence_after();
-            dec_tmem_ld<NQ>(tmem_s + lane_addr + st * 64, r);
-            tmem_ld_wait();
-            float sv[NQ], mx[NQ];
+        int k = 0, sg = 0;   // chunks, segments so far
+        for (long long u = u0; u < u1 && !failed; ++sg) {
+            const Seg g = segment(u);
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) { sv[q] = valid ? __uint_as_float(r[q]) * p.scale_log2 : -INFINITY; mx[q] = sv[q]; }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
-            if (lane < NQ) {   // lane q publishes the warp's maximum of query q
-                float v = mx[0];
-#pragma unroll
-                for (int q = 1; q < NQ; ++q) v = (lane == q) ? mx[q] : v;
-                wmax[t & 1][qd][lane] = v;
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&mx_full[t & 1]);
-            DC_FAIL_AT(13, !mbar_wait(&mx_full[t & 1], (t >> 1) & 1, lim));
-            // new running maxima (the same in every thread), factors for what is held relative to the old ones
-            float alpha[NQ];
-            unsigned char *pbase = p_smem + (size_t)st * DC_PBUF + (size_t)(j >> 6) * DC_QSLAB + (j & 7) * 2;
-            const int piece = (j & 63) >> 3;
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const float mc = fmaxf(fmaxf(wmax[t & 1][0][q], wmax[t & 1][1][q]), fmaxf(wmax[t & 1][2][q], wmax[t & 1][3][q]));
-                const float mn = fmaxf(m_run[q], mc);
-                alpha[q] = (m_run[q] == -INFINITY) ? 0.0f : fast_exp2(m_run[q] - mn);
-                m_run[q] = mn;
-                const float e = valid ? fast_exp2(sv[q] - mn) : 0.0f;
-                l_part[q] = fmaf(l_part[q], alpha[q], e);
-                // Pt as the K-major B operand [NQ rows x 128 keys]: row q, key j
-                *reinterpret_cast<uint16_t *>(pbase + (q >> 3) * 1024 + (q & 7) * 128 + ((piece ^ (q & 7)) << 4)) = pack_16(e, p.f16 != 0);
-            }
-            tc_fence_before();
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars.p_full[st]);
-            // Ot of the previous chunk was computed relative to the maxima before this update
-            if (t > 0) {
-                const int sp = (t - 1) & 1;
-                DC_FAIL_AT(9, !mbar_wait(&bars.o_full[sp], ((t - 1) >> 1) & 1, lim));
+            for (int q = 0; q < NQ; ++q) { m_run[q] = -INFINITY; l_part[q] = 0.0f; o_run[q] = 0.0f; }
+            for (int t = 0; t < g.n && !failed; ++t, ++k) {
+                const int st = k & 1;
+                const bool valid = (g.c0 + t) * DC_NK + j < p.Lk;
+                DC_FAIL_AT(8, !mbar_wait(&bars.s_full[st], (k >> 1) & 1, lim));
                 tc_fence_after();
-                dec_tmem_ld<NQ>(tmem_o + lane_addr + sp * 64, r);
+                dec_tmem_ld<NQ>(tmem_s + lane_addr + st * 64, r);
                 tmem_ld_wait();
+                float sv[NQ], mx[NQ];
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) o_run[q] = (o_run[q] + __uint_as_float(r[q])) * alpha[q];
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars.o_free[sp]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) o_run[q] *= alpha[q];
-            }
-        }
-        if (!failed) {
-            do {
-                const int sp = (n - 1) & 1;
-                DC_FAIL_AT(12, !mbar_wait(&bars.o_full[sp], ((n - 1) >> 1) & 1, lim));
-                tc_fence_after();
-                dec_tmem_ld<NQ>(tmem_o + lane_addr + sp * 64, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) o_run[q] += __uint_as_float(r[q]);
-                // row sums: over the 32 lanes, then over the four warps
+                for (int q = 0; q < NQ; ++q) { sv[q] = valid ? __uint_as_float(r[q]) * p.scale_log2 : -INFINITY; mx[q] = sv[q]; }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-                    for (int q = 0; q < NQ; ++q) l_part[q] += __shfl_xor_sync(0xffffffffu, l_part[q], o);
-                if (lane < NQ) {
-                    float v = l_part[0];
+                    for (int q = 0; q < NQ; ++q) mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
+                if (lane < NQ) {   // lane q publishes the warp's maximum of query q
+                    float v = mx[0];
 #pragma unroll
-                    for (int q = 1; q < NQ; ++q) v = (lane == q) ? l_part[q] : v;
-                    wsum[qd][lane] = v;
+                    for (int q = 1; q < NQ; ++q) v = (lane == q) ? mx[q] : v;
+                    wmax[st][qd][lane] = v;
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&sum_full);
-                DC_FAIL_AT(14, !mbar_wait(&sum_full, 0, lim));
-                if (d_active) {
+                if (lane == 0) mbar_arrive(&mx_full[st]);
+                DC_FAIL_AT(13, !mbar_wait(&mx_full[st], (k >> 1) & 1, lim));
+                // new running maxima (the same in every thread), factors for what is held relative to the old ones
+                float alpha[NQ];
+                unsigned char *pbase = p_smem + (size_t)st * DC_PBUF + (size_t)(j >> 6) * DC_QSLAB + (j & 7) * 2;
+                const int piece = (j & 63) >> 3;
 #pragma unroll
-                    for (int q = 0; q < NQ; ++q) {
-                        if (q >= p.Lq) break;
-                        const float l = (wsum[0][q] + wsum[1][q]) + (wsum[2][q] + wsum[3][q]);
-                        if (p.nsplit == 1) {
-                            reinterpret_cast<uint16_t *>(p.O)[(bh * p.Lq + q) * (long long)D + drow] = pack_16(o_run[q] / l, p.f16 != 0);
-                        } else {
-                            p.part_O[((bh * p.nsplit + split) * DC_MQ + q) * (long long)D + drow] = o_run[q];
-                            if (drow == 0) {
-                                float *pm = p.part_ml + ((bh * p.nsplit + split) * DC_MQ + q) * 2;
-                                pm[0] = m_run[q];
-                                pm[1] = l;
+                for (int q = 0; q < NQ; ++q) {
+                    const float mc = fmaxf(fmaxf(wmax[st][0][q], wmax[st][1][q]), fmaxf(wmax[st][2][q], wmax[st][3][q]));
+                    const float mn = fmaxf(m_run[q], mc);
+                    alpha[q] = (m_run[q] == -INFINITY) ? 0.0f : fast_exp2(m_run[q] - mn);
+                    m_run[q] = mn;
+                    const float e = valid ? fast_exp2(sv[q] - mn) : 0.0f;
+                    l_part[q] = fmaf(l_part[q], alpha[q], e);
+                    // Pt as the K-major B operand [NQ rows x 128 keys]: row q, key j
+                    *reinterpret_cast<uint16_t *>(pbase + (q >> 3) * 1024 + (q & 7) * 128 + ((piece ^ (q & 7)) << 4)) = pack_16(e, p.f16 != 0);
+                }
+                tc_fence_before();
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars.p_full[st]);
+                // Ot of the previous chunk was computed relative to the maxima before this update
+                if (t > 0) {
+                    const int sp = (k - 1) & 1;
+                    DC_FAIL_AT(9, !mbar_wait(&bars.o_full[sp], ((k - 1) >> 1) & 1, lim));
+                    tc_fence_after();
+                    dec_tmem_ld<NQ>(tmem_o + lane_addr + sp * 64, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) o_run[q] = (o_run[q] + __uint_as_float(r[q])) * alpha[q];
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars.o_free[sp]);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) o_run[q] *= alpha[q];
+                }
+            }
+            if (!failed) {
+                do {
+                    const int sp = (k - 1) & 1;
+                    DC_FAIL_AT(12, !mbar_wait(&bars.o_full[sp], ((k - 1) >> 1) & 1, lim));
+                    tc_fence_after();
+                    dec_tmem_ld<NQ>(tmem_o + lane_addr + sp * 64, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) o_run[q] += __uint_as_float(r[q]);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars.o_free[sp]);
+                    // row sums: over the 32 lanes, then over the four warps
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q) l_part[q] += __shfl_xor_sync(0xffffffffu, l_part[q], o);
+                    if (lane < NQ) {
+                        float v = l_part[0];
+#pragma unroll
+                        for (int q = 1; q < NQ; ++q) v = (lane == q) ? l_part[q] : v;
+                        wsum[qd][lane] = v;
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sum_full);
+                    DC_FAIL_AT(14, !mbar_wait(&sum_full, sg & 1, lim));
+                    const int first = dec_cta_of(p, g.bh * p.chunks), split = (int)blockIdx.x - first;
+                    const bool whole = g.n == p.chunks;   // the head is this CTA's alone
+                    if (d_active) {
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q) {
+                            if (q >= p.Lq) break;
+                            const float l = (wsum[0][q] + wsum[1][q]) + (wsum[2][q] + wsum[3][q]);
+                            if (whole) {
+                                reinterpret_cast<uint16_t *>(p.O)[(g.bh * p.Lq + q) * (long long)D + drow] = pack_16(o_run[q] / l, p.f16 != 0);
+                            } else {
+                                p.part_O[((g.bh * p.nsplit + split) * DC_MQ + q) * (long long)D + drow] = o_run[q];
+                                if (drow == 0) {
+                                    float *pm = p.part_ml + ((g.bh * p.nsplit + split) * DC_MQ + q) * 2;
+                                    pm[0] = m_run[q];
+                                    pm[1] = l;
+                                }
                             }
                         }
                     }
-                }
-            } while (false);
+                } while (false);
+            }
+            u += g.n;
         }
     } else if (p.rotate_q || p.rotate_k) {
         const int tid = threadIdx.x - 6 * 32;
-        do {
+        int k = 0, sg = 0;
+        for (long long u = u0; u < u1 && !failed; ++sg) {
+            const Seg g = segment(u);
             if (p.rotate_q) {
-                DC_FAIL_AT(10, !dec_encode_tile(q_smem, DC_MQ, DC_QSLAB, nch, D, 0, p.table_kind, p.sinus != 0, p.tab, tid,
-                                                [&]() { return mbar_wait(&bars.q_full, 0, lim); }));
+                const int qb = sg & 1;
+                DC_FAIL_AT(10, !dec_encode_tile(q_smem + qb * q_buf, DC_MQ, DC_QSLAB, nch, D, 0, p.table_kind, p.sinus != 0, p.tab, tid,
+                                                [&]() { return mbar_wait(&q_full[qb], (sg >> 1) & 1, lim); }));
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&bars.q_ready);
+                if (lane == 0) mbar_arrive(&q_ready[qb]);
             }
             if (p.rotate_k) {
-                for (int t = 0; t < n; ++t) {
-                    const int st = t & 1;
-                    DC_FAIL_AT(11, !dec_encode_tile(k_smem + (size_t)st * kv_stage, DC_NK, DC_KSLAB, nch, D, (c0 + t) * DC_NK, p.table_kind, p.sinus != 0, p.tab, tid,
-                                                    [&]() { return mbar_wait(&bars.k_full[st], (t >> 1) & 1, lim); }));
+                for (int t = 0; t < g.n; ++t, ++k) {
+                    const int st = k & 1;
+                    DC_FAIL_AT(11, !dec_encode_tile(k_smem + (size_t)st * kv_stage, DC_NK, DC_KSLAB, nch, D, (g.c0 + t) * DC_NK, p.table_kind, p.sinus != 0, p.tab, tid,
+                                                    [&]() { return mbar_wait(&bars.k_full[st], (k >> 1) & 1, lim); }));
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bars.k_ready[st]);
                 }
             }
-        } while (false);
+            u += g.n;
+        }
     }
 
     if (failed) for (int i = 0; i < 2000; ++i) __nanosleep(1000);
@@ -668,15 +713,17 @@ __global__ void dec_combine_kernel(const DecParams p) {
     grid_dependency_wait();
     const int i = blockIdx.x;
     const long long bh = blockIdx.y;
+    const int ns = p.ctas ? dec_cta_of(p, (bh + 1) * p.chunks - 1) - dec_cta_of(p, bh * p.chunks) + 1 : p.nsplit;
+    if (p.ctas && ns == 1) return;   // written by the CTA that had the whole head
     const float *ml = p.part_ml + (bh * p.nsplit * DC_MQ + i) * 2;
     float m = -INFINITY;
-    for (int s = 0; s < p.nsplit; ++s) m = fmaxf(m, ml[(long long)s * DC_MQ * 2]);
+    for (int s = 0; s < ns; ++s) m = fmaxf(m, ml[(long long)s * DC_MQ * 2]);
     float l = 0.0f;
-    for (int s = 0; s < p.nsplit; ++s) l += fast_exp2(ml[(long long)s * DC_MQ * 2] - m) * ml[(long long)s * DC_MQ * 2 + 1];
+    for (int s = 0; s < ns; ++s) l += fast_exp2(ml[(long long)s * DC_MQ * 2] - m) * ml[(long long)s * DC_MQ * 2 + 1];
     const float inv = 1.0f / l;
     for (int d = 2 * threadIdx.x; d < p.D; d += 2 * blockDim.x) {
         float o0 = 0.0f, o1 = 0.0f;
-        for (int s = 0; s < p.nsplit; ++s) {
+        for (int s = 0; s < ns; ++s) {
             const float w = fast_exp2(ml[(long long)s * DC_MQ * 2] - m);
             const float2 v = *reinterpret_cast<const float2 *>(p.part_O + ((bh * p.nsplit + s) * DC_MQ + i) * (long long)p.D + d);
             o0 = fmaf(w, v.x, o0);
@@ -744,6 +791,19 @@ inline int dec_run(const b200attn_args &a, int rd, float base, TcwScratch &sc, T
     if (nsplit < 1) nsplit = 1;
     p.cps = (total_chunks + nsplit - 1) / nsplit;
     p.nsplit = (total_chunks + p.cps - 1) / p.cps;   // no empty split
+    p.chunks = total_chunks;
+    const bool transposed = Lq <= 32;
+    if (transposed) {
+        // All chunks over the SMs, at least two each, where that shortens the longest CTA by enough chunks (some 2 us each) to pay for the
+        // hand-over at a head's end and, where heads were whole, the combine launch: 128 heads, 2000 keys, 16 -> 14 chunks, took 35.4 us
+        // shared out and 32.9 us as whole heads; 75 heads, 4000 keys, 32 -> 17: 44.4 and 59.1 us.  Beyond two heads per SM: whole heads.
+        const long long T = BH * total_chunks, splits = p.nsplit, whole = BH * splits;
+        const long long even = (T + 1) / 2 < sm_count ? (T + 1) / 2 : sm_count;
+        const long long saved = p.cps * ((whole + sm_count - 1) / sm_count) - (T + even - 1) / even;
+        const long long ctas = BH > 2LL * sm_count || saved < (splits == 1 ? 4 : 2) ? whole : even;
+        p.ctas = (int)ctas;
+        p.nsplit = T % ctas == 0 && (T / ctas) % total_chunks == 0 ? 1 : (int)((total_chunks - 1) / (T / ctas) + 2);   // CTAs a head can meet
+    }
     p.scale_log2 = 1.4426950408889634f / sqrtf((float)D);
     p.rotate_q = a.pe != B200ATTN_PE_NONE ? 1 : 0;
     p.rotate_k = pe_encodes_k(a.pe) ? 1 : 0;
@@ -781,8 +841,8 @@ inline int dec_run(const b200attn_args &a, int rd, float base, TcwScratch &sc, T
         snprintf(t_tc_error, sizeof t_tc_error, "cuTensorMapEncodeTiled failed");
         return B200ATTN_ERR_CUDA;
     }
-    const dim3 grid((unsigned)p.nsplit, (unsigned)BH);
-    const size_t smem = dec_smem_bytes(nch);
+    const dim3 grid(transposed ? (unsigned)p.ctas : (unsigned)p.nsplit, transposed ? 1u : (unsigned)BH);
+    const size_t smem = dec_smem_bytes(nch) + (transposed ? (size_t)nch * DC_QSLAB : 0);
     // up to 32 queries: the transposed kernel (keys along the tensor-memory lanes); more: a row per query
     if (Lq <= 16) { if (nch == 1) launch_dependent(dec_t_kernel<1, 16>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); else launch_dependent(dec_t_kernel<2, 16>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); }
     else if (Lq <= 32) { if (nch == 1) launch_dependent(dec_t_kernel<1, 32>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); else launch_dependent(dec_t_kernel<2, 32>, grid, DC_THREADS, smem, 1, st, tmQ, tmK, tmV, p); }
