@@ -728,7 +728,8 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
         }
     }
     if (!done && !(a->flags & (B200ATTN_FLAG_FORCE_GENERIC | B200ATTN_FLAG_FORCE_TWO_PASS)) && f32tc_supported(*a)) {
-        // (against the two FFMA launches 1.6 times faster at 5 heads, 65 x 64, head_d 1, 2.1 at one head, 80 x 80, 8.9 at 2 heads, 2048 x 2048, 12 at 2 heads, 300 x 2000)
+        // (against the two FFMA launches 1.6 times faster at 5 heads, 65 x 64, head_d 1, 2.1 at one head, 80 x 80, 8.9 at 2 heads, 2048 x 2048, 12 at 2 heads, 300 x 2000; 16 bit 1.1 times at
+        // one head, 1 x 66, head_d 16, 1.4 at 148 heads, 64 x 65, head_d 248, 5.7 at 32 heads, 777 x 1000, head_d 96, 18 at one head, 4 x 8192, head_d 96)
         rc = f32tc_run(*a, rd, base, c->f32, c->err_dev, c->err_host_dev, c->sm_count, current_spin_limit(), (size_t)g_score_scratch_mb.load() << 20, st, &g_launches);
         if (rc == B200ATTN_OK) { t_last_path = "tc_f32"; done = true; }
         else if (rc != -1) return fail(rc, "%s", tc_bf16_error());

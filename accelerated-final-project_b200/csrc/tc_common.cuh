@@ -433,19 +433,6 @@ inline bool make_tmap_grouped_heads(CUtensorMap *m, const void *base, long long 
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// `heads` matrices of [rows][cols] 16-bit elements, cols a multiple of 8 only, as [cols][rows][heads] with a box of one
-// 64-column group: rows beyond a head's last and columns beyond a row's end read as zero.
-inline bool make_tmap_cols_heads(CUtensorMap *m, const void *base, long long heads, long long rows, long long cols, int box_rows) {
-    PFN_tmapEncodeTiled enc = tmap_encode_fn();
-    if (!enc || cols % 8 != 0) return false;
-    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)heads};
-    cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)rows * (cuuint64_t)cols * 2};
-    cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

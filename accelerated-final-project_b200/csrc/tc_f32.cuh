@@ -1,12 +1,17 @@
-// fp32 attention forward for sequences longer than 64 on the tensor cores, at fp32 accuracy.
+// Attention forward for sequences longer than 64 on the tensor cores, at fp32 accuracy: fp32 tensors, and 16-bit tensors of the
+// head widths that the 16-bit kernels do not take (no multiple of 64; 192 with an encoding).
 //
 // An fp32 value is cut into three bf16 pieces x = x1 + x2 + x3 (8 significant bits each: the sum is exact), and a product
 // a b is taken as a1 b1 + (a1 b2 + a2 b1) + (a1 b3 + a2 b2 + a3 b1): what is left out is below 2^-23 |a b| (about 2^-25 on
 // average).  Six bf16 MMAs cost what three tf32 MMAs on a hi / lo pair cost and keep two more bits.  The leading products
 // have an accumulator of their own and are added to the small ones in fp32 by the thread that reads them, and P V starts a
-// fresh accumulator per 128 keys, summed in registers: the chain of roundings at the full magnitude is as short as
-// head_d / 16 and len_k / 128.  (Replaces, for these shapes, the FFMA kernels of splitd.cuh; same mathematics as the
+// fresh accumulator per 64 keys, summed in registers: the chain of roundings at the full magnitude is as short as
+// head_d / 16 and len_k / 64.  (Replaces, for these shapes, the FFMA kernels of splitd.cuh; same mathematics as the
 // reference's fp32 kernel, final/attention.cu:84-191: softmax statistics, probabilities and sums are fp32.)
+// A 16-bit tensor is fewer pieces (bf16 one, fp16 two, an encoded Q or K three) and its result is rounded once, at the end.  The 16-bit
+// kernel of tc_fa.cuh at these widths (P and encoded operands rounded to 16 bits) was no replacement for the CUDA-core kernels, which
+// hold both in fp32: 2 x 16 heads, 777 x 1000, head_d 96, bf16, its output lay 2.5e-3 from theirs; this one lies 5e-5 from it (a result
+// in some thousands rounds the other way), in 126 us against 717 us on the CUDA cores and 22 us there.
 //
 //   f32_split_kernel    Q, K, V -> three bf16 planes each, columns padded to whole groups of 64 with zeros; a positional
 //                       encoding is applied here, once per element, with the fp32 arithmetic of the reference tables;
@@ -25,15 +30,19 @@
 // Every wait is bounded.
 #pragma once
 
+#include <type_traits>
+
 #include "tc_bf16.cuh"
 
 namespace b200attn {
 
 constexpr int F3_T = 128;                    // queries and keys per tile
 constexpr int F3_SLAB = F3_T * 128;          // [128 rows x 64 bf16]: one plane of a 64-column chunk
-constexpr int F3_STAGE = 6 * F3_SLAB;        // score kernel: Q1 Q2 Q3 K1 K2 K3
+// score kernel, operands of `nq` pieces: a stage is the planes of Q, then those of K; fewer pieces, more stages
+__host__ __device__ constexpr int f3_stage(int nq) { return 2 * nq * F3_SLAB; }
+__host__ __device__ constexpr int f3_stages(int nq) { return nq == 3 ? 2 : nq == 2 ? 3 : 4; }
 constexpr int F3_VSLAB = 64 * 128;           // [64 keys x 64 bf16]
-constexpr int F3_VSTAGE = 3 * F3_VSLAB;      // P V kernel: V1 V2 V3 of 64 keys x 64 columns
+constexpr int F3_VSTAGE = 3 * F3_VSLAB;      // P V kernel: the pieces of V of 64 keys x 64 columns
 constexpr int F3_SSTEP = 64 * F3_T * 4;      // scores of 64 keys as the score kernel leaves them
 constexpr int F3_PBUF = 3 * F3_SLAB;         // P1 P2 P3 [128 rows x 64 keys]
 constexpr int F3_A_THREADS = 576;            // score kernel: warp 0 loads, warp 1 issues, warps 2-17 four threads per query row
@@ -47,11 +56,11 @@ struct F32Params {
     int nq, nk, ndb;           // query tiles, key tiles, blocks of 64 output columns
     int upc;                   // P V kernel: steps of 64 keys per CTA of the cluster
     float c;                   // log2(e) / sqrt(head_d)
-    const __nv_bfloat16 *q, *k, *v;   // planes [3][heads][L][Dp]
+    const __nv_bfloat16 *q, *k, *v;   // planes [pieces][heads][L][Dp]
     float *S;                  // [heads][nq][nk][32 groups of 4 keys][128 rows][4]
     int *rowmax;               // [heads][nq * 128] largest score of a row, as f3_key; the split kernel starts it at the lowest key
-    float *O;                  // [heads * Lq][D]
-    int vec_out;               // 16-byte output stores
+    void *O;                   // [heads * Lq][D]
+    int vec_out;               // stores of four columns
     const unsigned *mark;      // == call: a non-finite value has been met
     unsigned call;
     unsigned *err, *err_sys;
@@ -69,17 +78,22 @@ __device__ __forceinline__ void f3_split2(float x0, float x1, uint32_t &a, uint3
 // fp32 values as integers of the same order (NaN aside), and back
 __device__ __forceinline__ int f3_key(float x) { const int i = __float_as_int(x); return i >= 0 ? i : i ^ 0x7fffffff; }
 __device__ __forceinline__ float f3_unkey(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
-// the value back from its pieces
-__device__ __forceinline__ float f3_join(const __nv_bfloat16 *p, long long plane) {
-    return (__bfloat162float(p[0]) + __bfloat162float(p[plane])) + __bfloat162float(p[2 * plane]);
+// the value back from its N pieces
+template <int N> __device__ __forceinline__ float f3_join(const __nv_bfloat16 *p, long long plane) {
+    float x = __bfloat162float(p[0]);
+    if (N > 1) x += __bfloat162float(p[plane]);
+    if (N > 2) x += __bfloat162float(p[2 * plane]);
+    return x;
 }
 
 // ---- split (and encode) ---------------------------------------------------------------------------
 struct F32SplitTensor {
-    const float *X;
-    __nv_bfloat16 *Y;          // [3][heads][L][Dp]
+    const void *X;
+    __nv_bfloat16 *Y;          // [pieces][heads][L][Dp]
     int L;
     int encode;                // the encoding applies to this tensor
+    int pieces;
+    int track;                 // its non-finite values must not reach the MMAs (with one piece on either side they may)
 };
 struct F32SplitParams {
     F32SplitTensor t[3];       // blockIdx.z
@@ -95,14 +109,16 @@ struct F32SplitParams {
 
 // A thread owns eight columns of one row position and takes a share (gridDim.y) of the heads with them, so that the angles
 // are computed once per share; the loads of two heads are in flight together.
+template <typename T>
 __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) {
     grid_launch_dependents();
     grid_dependency_wait();
-    const F32SplitTensor T = p.t[blockIdx.z];
+    const F32SplitTensor t = p.t[blockIdx.z];
+    const T *X = reinterpret_cast<const T *>(t.X);
     const int ng = p.Dp >> 3, D = p.D;
-    const long long total = (long long)T.L * ng, slab = (long long)T.L * D, yslab = (long long)T.L * p.Dp, plane = yslab * p.heads;
+    const long long total = (long long)t.L * ng, slab = (long long)t.L * D, yslab = (long long)t.L * p.Dp, plane = yslab * p.heads;
     const bool sinus = p.pe == PE_SINUSOIDAL, half = pe_pairs_halves(p.pe);
-    const bool vec = (D & 3) == 0 && (reinterpret_cast<uintptr_t>(T.X) & 15) == 0;
+    const bool vec = D % (16 / (int)sizeof(T)) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     const int step = gridDim.y;
     bool odd = false;   // a non-finite value has been met
     if (blockIdx.z == 0)
@@ -111,7 +127,7 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
     for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long long)gridDim.x * blockDim.x) {
         const int l = (int)(w / ng), d0 = (int)(w - (long long)l * ng) * 8;
         const int n = min(8, D - d0);            // real columns, <= 0 in the padding
-        const bool enc = T.encode && n > 0 && (sinus || d0 < p.rd);
+        const bool enc = t.encode && n > 0 && (sinus || d0 < p.rd);
         float cs[8], sn[8];   // per column (interleaved pairs: the two columns of a pair share theirs)
         if (enc) {
 #pragma unroll
@@ -132,13 +148,17 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
             }
         }
         auto load = [&](int h, float (&x)[8]) {
-            const float *xp = T.X + h * slab + (long long)l * D + d0;
+            const T *xp = X + h * slab + (long long)l * D + d0;
             if (vec && n == 8) {
-                const float4 a = *reinterpret_cast<const float4 *>(xp), b = *reinterpret_cast<const float4 *>(xp + 4);
-                x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+                uint4 raw[sizeof(T) / 2];
+#pragma unroll
+                for (int i = 0; i < (int)sizeof(T) / 2; ++i) raw[i] = reinterpret_cast<const uint4 *>(xp)[i];
+                const T *e8 = reinterpret_cast<const T *>(raw);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = to_f32(e8[e]);
             } else {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] = e < n ? xp[e] : 0.0f;
+                for (int e = 0; e < 8; ++e) x[e] = e < n ? to_f32(xp[e]) : 0.0f;
             }
         };
         auto store = [&](int h, float (&x)[8]) {
@@ -148,13 +168,13 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
                     for (int e = 0; e < 8; ++e)
                         if (e < n) x[e] += (e & 1) ? cs[e] : sn[e];
                 } else if (half) {
-                    const float *xr = T.X + h * slab + (long long)l * D;
+                    const T *xr = X + h * slab + (long long)l * D;
                     const int hr = p.rd >> 1;
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
                         const int d = d0 + e;
-                        if (d < hr) x[e] = x[e] * cs[e] - xr[d + hr] * sn[e];
-                        else if (d < p.rd) x[e] = xr[d - hr] * sn[e] + x[e] * cs[e];
+                        if (d < hr) x[e] = x[e] * cs[e] - to_f32(xr[d + hr]) * sn[e];
+                        else if (d < p.rd) x[e] = to_f32(xr[d - hr]) * sn[e] + x[e] * cs[e];
                     }
                 } else {
 #pragma unroll
@@ -172,15 +192,15 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
 #pragma unroll
             for (int e = 0; e < 8; ++e)
                 if ((__float_as_uint(x[e]) & 0x7f800000u) == 0x7f800000u) {   // the value in the first piece (a NaN stays one), zero in the others
-                    odd = true;
+                    odd = odd || t.track;
                     const uint32_t keep = (e & 1) ? 0x0000ffffu : 0xffff0000u;
                     b[e >> 1] &= keep; c[e >> 1] &= keep;
                     if (x[e] != x[e]) a[e >> 1] |= (e & 1) ? 0x00400000u : 0x00000040u;
                 }
-            __nv_bfloat16 *yp = T.Y + h * yslab + (long long)l * p.Dp + d0;
+            __nv_bfloat16 *yp = t.Y + h * yslab + (long long)l * p.Dp + d0;
             *reinterpret_cast<uint4 *>(yp) = make_uint4(a[0], a[1], a[2], a[3]);
-            *reinterpret_cast<uint4 *>(yp + plane) = make_uint4(b[0], b[1], b[2], b[3]);
-            *reinterpret_cast<uint4 *>(yp + 2 * plane) = make_uint4(c[0], c[1], c[2], c[3]);
+            if (t.pieces > 1) *reinterpret_cast<uint4 *>(yp + plane) = make_uint4(b[0], b[1], b[2], b[3]);
+            if (t.pieces > 2) *reinterpret_cast<uint4 *>(yp + 2 * plane) = make_uint4(c[0], c[1], c[2], c[3]);
         };
         for (int h = blockIdx.y; h < p.heads; h += 2 * step) {
             float x0[8], x1[8];
@@ -215,17 +235,20 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
 // small ones apart, and the epilogue warps add the groups of a tile up in registers while the next group is multiplied.  (The
 // groups also keep the chain short in which the tensor core cuts sums off, always towards zero: with one accumulator over
 // head_d 512 the output erred by 7.8e-7 against 64 bits on normal inputs, with groups of 128 by 2.1e-7; the FFMA kernels: 4.1e-7.)
+template <int NQ>   // pieces of Q and K
 __global__ void __launch_bounds__(F3_A_THREADS, 1)
 f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const F32Params p) {
+    constexpr int STAGE = f3_stage(NQ), NST = f3_stages(NQ);
     extern __shared__ unsigned char f3_smem_raw[];
-    __shared__ uint64_t full[2], empty[2], acc_full[2], acc_empty[2];
+    __shared__ uint64_t full[NST], empty[NST], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     unsigned char *smem = f3_smem_raw + ((1024u - (smem_u32(f3_smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nch = p.Dp >> 6, per_head = p.nq * p.nk, tiles = per_head * p.heads;
     const uint32_t lim = p.spin_limit;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 16); }
+        for (int i = 0; i < NST; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 16); }
         mbar_fence_init();
         tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK);
     }
@@ -249,14 +272,14 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                 const int h = tile / per_head, r = tile - h * per_head, qt = r / p.nk, kt = r - qt * p.nk;
                 for (int ch = 0; ch < nch; ++ch) {
                     F3_FAIL_AT(0, !mbar_wait(&empty[s], (uint32_t)ph ^ 1u, lim));
-                    unsigned char *st = smem + (size_t)s * F3_STAGE;
-                    mbar_expect_tx(&full[s], F3_STAGE);
+                    unsigned char *st = smem + (size_t)s * STAGE;
+                    mbar_expect_tx(&full[s], STAGE);
 #pragma unroll
-                    for (int i = 0; i < 3; ++i) {
+                    for (int i = 0; i < NQ; ++i) {
                         tma_load_4d(st + i * F3_SLAB, &tmQ, 0, qt * F3_T, ch, i * p.heads + h, &full[s]);
-                        tma_load_4d(st + (3 + i) * F3_SLAB, &tmK, 0, kt * F3_T, ch, i * p.heads + h, &full[s]);
+                        tma_load_4d(st + (NQ + i) * F3_SLAB, &tmK, 0, kt * F3_T, ch, i * p.heads + h, &full[s]);
                     }
-                    ph ^= s; s ^= 1;
+                    if (++s == NST) { s = 0; ph ^= 1; }
                 }
             }
         }
@@ -271,22 +294,22 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                     if (first) F3_FAIL_AT(1, !mbar_wait(&acc_empty[g & 1], ((g >> 1) & 1) ^ 1u, lim));
                     F3_FAIL_AT(1, !mbar_wait(&full[s], (uint32_t)ph, lim));
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + (size_t)s * F3_STAGE), ta = tmem + 256u * (g & 1);
-                    const uint64_t q1 = umma_desc_k_sw128(sa), k1 = umma_desc_k_sw128(sa + 3 * F3_SLAB);
+                    const uint32_t sa = smem_u32(smem + (size_t)s * STAGE), ta = tmem + 256u * (g & 1);
+                    const uint64_t q1 = umma_desc_k_sw128(sa), k1 = umma_desc_k_sw128(sa + NQ * F3_SLAB);
                     constexpr uint64_t PL = F3_SLAB >> 4;   // from a plane to the next, in descriptor units
                     // (one accumulator after the other: an MMA waits for the one before it where their columns overlap in part)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_bf16(ta, q1 + 2 * k, k1 + 2 * k, id256, (!first || k != 0) ? 1u : 0u);   // Q1 [K1; K2]
+                    for (int k = 0; k < 4; ++k) umma_bf16(ta, q1 + 2 * k, k1 + 2 * k, NQ > 1 ? id256 : id128, (!first || k != 0) ? 1u : 0u);   // Q1 [K1; K2]
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        umma_bf16(ta + 128, q1 + PL + 2 * k, k1 + 2 * k, id128, 1u);                  // Q2 K1
-                        umma_bf16(ta + 128, q1 + 2 * k, k1 + 2 * PL + 2 * k, id128, 1u);              // Q1 K3
-                        umma_bf16(ta + 128, q1 + PL + 2 * k, k1 + PL + 2 * k, id128, 1u);             // Q2 K2
-                        umma_bf16(ta + 128, q1 + 2 * PL + 2 * k, k1 + 2 * k, id128, 1u);              // Q3 K1
+                        if (NQ > 1) umma_bf16(ta + 128, q1 + PL + 2 * k, k1 + 2 * k, id128, 1u);      // Q2 K1
+                        if (NQ > 2) umma_bf16(ta + 128, q1 + 2 * k, k1 + 2 * PL + 2 * k, id128, 1u);  // Q1 K3
+                        if (NQ > 1) umma_bf16(ta + 128, q1 + PL + 2 * k, k1 + PL + 2 * k, id128, 1u); // Q2 K2
+                        if (NQ > 2) umma_bf16(ta + 128, q1 + 2 * PL + 2 * k, k1 + 2 * k, id128, 1u);  // Q3 K1
                     }
                     umma_commit(&empty[s]);
                     if (!first || ch + 1 == nch) { umma_commit(&acc_full[g & 1]); ++g; }
-                    ph ^= s; s ^= 1;
+                    if (++s == NST) { s = 0; ph ^= 1; }
                 }
             }
         }
@@ -310,7 +333,7 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         if (j < valid)
-                            for (int d = 0; d < p.D; ++d) s[j] = fmaf(f3_join(qp + d, qpl), f3_join(kp + (long long)j * p.Dp + d, kpl), s[j]);
+                            for (int d = 0; d < p.D; ++d) s[j] = fmaf(f3_join<NQ>(qp + d, qpl), f3_join<NQ>(kp + (long long)j * p.Dp + d, kpl), s[j]);
                 }
             } else {
                 for (int c = 0; c < nch; c += 2, ++g) {
@@ -321,10 +344,10 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                     for (int i = 0; i < 2; ++i) {
                         uint32_t a[16], b[16];
                         tmem_ld16(ta + 16 * i, a);
-                        tmem_ld16(ta + 128 + 16 * i, b);
+                        if (NQ > 1) tmem_ld16(ta + 128 + 16 * i, b);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) s[16 * i + j] += __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                        for (int j = 0; j < 16; ++j) s[16 * i + j] += NQ > 1 ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -376,6 +399,7 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
 // that collect the products of one order of magnitude (1, 2^-8, 2^-16).  A set adds the accumulators of its step up and
 // folds them into its running output (32 registers a thread) before it hands over the next P; the exponentials of that P
 // are computed before it waits.  (Scores through shared memory: loaded into registers a step ahead they cost a step their latency.)
+template <typename T, int NV>   // the result's type, pieces of V
 __global__ void __launch_bounds__(F3_B_THREADS, 1)
 f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
     extern __shared__ unsigned char f3_smem_raw[];
@@ -433,14 +457,14 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
                 const int b = u & 1;
                 F3_FAIL_AT(0, !mbar_wait(&v_empty[b], (uint32_t)((u >> 1) & 1) ^ 1u, lim));
                 unsigned char *st = v_smem + (size_t)b * F3_VSTAGE;
-                mbar_expect_tx(&v_full[b], F3_VSTAGE);
+                mbar_expect_tx(&v_full[b], NV * F3_VSLAB);
 #pragma unroll
-                for (int i = 0; i < 3; ++i) tma_load_4d(st + i * F3_VSLAB, &tmV, 0, (u0 + u) * 64, db, i * p.heads + h, &v_full[b]);
+                for (int i = 0; i < NV; ++i) tma_load_4d(st + i * F3_VSLAB, &tmV, 0, (u0 + u) * 64, db, i * p.heads + h, &v_full[b]);
             }
         }
     } else if (warp == 1) {
         if (!plain && elect_one()) {
-            const uint32_t id1 = umma_idesc_bf16(128, 192, 0, 1), id2 = umma_idesc_bf16(128, 128, 0, 1), id3 = umma_idesc_bf16(128, 64, 0, 1);
+            const uint32_t id192 = umma_idesc_bf16(128, 192, 0, 1), id128 = umma_idesc_bf16(128, 128, 0, 1), id64 = umma_idesc_bf16(128, 64, 0, 1);
             for (int u = 0; u < n; ++u) {
                 const int b = u & 1;
                 const uint32_t par = (uint32_t)((u >> 1) & 1);
@@ -452,11 +476,15 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
                 // (one set of columns after the other: an MMA waits for the one before it where their columns overlap in part)
                 const uint64_t vd = umma_desc_mn_sw128(va, F3_VSLAB);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_bf16(to, pa + 2 * k, vd + 128 * k, id1, k != 0);
+                for (int k = 0; k < 4; ++k) umma_bf16(to, pa + 2 * k, vd + 128 * k, NV == 3 ? id192 : NV == 2 ? id128 : id64, k != 0);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_bf16(to + 64, pa + (F3_SLAB >> 4) + 2 * k, vd + 128 * k, id2, 1u);
+                for (int k = 0; k < 4; ++k) umma_bf16(to + 64, pa + (F3_SLAB >> 4) + 2 * k, vd + 128 * k, NV == 3 ? id128 : id64, NV > 1 || k != 0);
+                if (NV == 2) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_bf16(to + 128, pa + 2 * (F3_SLAB >> 4) + 2 * k, vd + 128 * k, id3, 1u);
+                    for (int k = 0; k < 4; ++k) umma_bf16(to + 128, pa + (F3_SLAB >> 4) + 2 * k, vd + (F3_VSLAB >> 4) + 128 * k, id64, k != 0);   // P2 V2
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) umma_bf16(to + 128, pa + 2 * (F3_SLAB >> 4) + 2 * k, vd + 128 * k, id64, NV > 1 || k != 0);
                 umma_commit(&v_empty[b]);
                 umma_commit(&pv_done[b]);
             }
@@ -476,7 +504,7 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
                         const __nv_bfloat16 *vp = p.v + ((long long)h * p.Lk + (u0 + u) * 64 + j) * p.Dp + db * 64 + 32 * hf;
                         if (hf == 0) l += e;
 #pragma unroll
-                        for (int d = 0; d < 32; ++d) o[d] = fmaf(e, f3_join(vp + d, vpl), o[d]);
+                        for (int d = 0; d < 32; ++d) o[d] = fmaf(e, f3_join<NV>(vp + d, vpl), o[d]);
                     }
             }
         } else {
@@ -572,13 +600,18 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
             }
             const float inv = 1.0f / sum;
             v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
-            float *op = p.O + ((long long)h * p.Lq + qrow) * p.D + db * 64 + c;
-            if (p.vec_out) *reinterpret_cast<float4 *>(op) = v;
-            else {
-                op[0] = v.x;
-                if (c + 1 < w) op[1] = v.y;
-                if (c + 2 < w) op[2] = v.z;
-                if (c + 3 < w) op[3] = v.w;
+            T *op = reinterpret_cast<T *>(p.O) + ((long long)h * p.Lq + qrow) * p.D + db * 64 + c;
+            if (p.vec_out) {
+                if constexpr (sizeof(T) == 4) *reinterpret_cast<float4 *>(op) = v;
+                else {
+                    constexpr bool H = std::is_same<T, __half>::value;
+                    *reinterpret_cast<uint2 *>(op) = make_uint2(pack_16x2(v.x, v.y, H), pack_16x2(v.z, v.w, H));
+                }
+            } else {
+                op[0] = OutCvt<T>::one(v.x);
+                if (c + 1 < w) op[1] = OutCvt<T>::one(v.y);
+                if (c + 2 < w) op[2] = OutCvt<T>::one(v.z);
+                if (c + 3 < w) op[3] = OutCvt<T>::one(v.w);
             }
         }
     }
@@ -595,7 +628,7 @@ struct F32Scratch {   // per device, grown on demand
     size_t bytes = 0;
     unsigned *mark = nullptr;
     unsigned calls = 0;
-    bool attr = false;
+    bool attr[3] = {};   // fp32, fp16, bf16
     void release() {
         if (buf) cudaFree(buf);
         if (mark) cudaFree(mark);
@@ -604,24 +637,35 @@ struct F32Scratch {   // per device, grown on demand
 };
 
 inline bool f32tc_supported(const b200attn_args &a) {
-    return a.dtype == B200ATTN_F32 && (a.len_q > 64 || a.len_k > 64) && a.head_d <= 512;
+    if (a.len_q <= 64 && a.len_k <= 64) return false;
+    if (a.dtype == B200ATTN_F32) return a.head_d <= 512;
+    // 16 bit: the widths up to 256 whose 16-bit kernels would round what the CUDA-core kernels hold in fp32
+    if (a.head_d % 8 != 0 || a.head_d > 256 || (a.head_d % 64 == 0 && (a.head_d != 192 || a.len_q <= 64))) return false;
+    return (((uintptr_t)a.Q | (uintptr_t)a.K | (uintptr_t)a.V | (uintptr_t)a.out) & 15) == 0;
 }
 
 // Returns B200ATTN_OK, -1 when the shape should run on another path (also when the scratch could not be allocated: nothing
 // has been launched then), or a status with tc_bf16_error() set.
-inline int f32tc_run(const b200attn_args &a, int rd, float base, F32Scratch &sc, unsigned *err_dev, unsigned *err_sys, int sm_count, unsigned spin_limit,
+template <typename T>
+inline int f32tc_launch(const b200attn_args &a, int rd, float base, F32Scratch &sc, unsigned *err_dev, unsigned *err_sys, int sm_count, unsigned spin_limit,
                      size_t scratch_cap, cudaStream_t st, std::atomic<unsigned long long> *launches) {
     const long long BH = (long long)a.batch_sz * a.num_heads;
     const int Lq = a.len_q, Lk = a.len_k, D = a.head_d;
-    const size_t smem_a = 2 * (size_t)F3_STAGE + 1024, smem_b = 2 * (size_t)(F3_PBUF + F3_VSTAGE + F3_SSTEP) + 1024;
-    if (!sc.attr) {
-        if (cudaFuncSetAttribute(f32_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a) != cudaSuccess ||
-            cudaFuncSetAttribute(f32_pv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) != cudaSuccess) {
+    // pieces that make up a value: of V, and of Q and K (fp32 values once encoded)
+    constexpr int NV = sizeof(T) == 4 ? 3 : std::is_same<T, __half>::value ? 2 : 1;
+    const int nqp = a.pe != B200ATTN_PE_NONE ? 3 : NV;
+    auto smem_a = [](int n) { return f3_stages(n) * (size_t)f3_stage(n) + 1024; };
+    const size_t smem_b = 2 * (size_t)(F3_PBUF + F3_VSTAGE + F3_SSTEP) + 1024;
+    const int type = sizeof(T) == 4 ? 0 : std::is_same<T, __half>::value ? 1 : 2;
+    if (!sc.attr[type]) {
+        if (cudaFuncSetAttribute(f32_scores_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a(NV)) != cudaSuccess ||
+            cudaFuncSetAttribute(f32_scores_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a(3)) != cudaSuccess ||
+            cudaFuncSetAttribute(f32_pv_kernel<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) != cudaSuccess) {
             (void)cudaGetLastError();
             snprintf(t_tc_error, sizeof t_tc_error, "cudaFuncSetAttribute(max dynamic shared memory) failed");
             return B200ATTN_ERR_CUDA;
         }
-        sc.attr = true;
+        sc.attr[type] = true;
     }
     F32Params p{};
     p.Lq = Lq; p.Lk = Lk; p.D = D; p.Dp = (D + 63) & ~63;
@@ -629,8 +673,8 @@ inline int f32tc_run(const b200attn_args &a, int rd, float base, F32Scratch &sc,
     if (nq * nk >= (1ll << 30) || nq * ndb > 65535) return -1;
     p.nq = (int)nq; p.nk = (int)nk; p.ndb = (int)ndb;
     // a pass takes as many heads as the scratch cap has room for
-    const size_t qb = (size_t)Lq * p.Dp * 6, kb = (size_t)Lk * p.Dp * 6, sb = (size_t)nq * nk * F3_T * F3_T * 4, tb = (size_t)nq * F3_T * 4;
-    const size_t per_head = qb + 2 * kb + sb + tb;
+    const size_t qb = (size_t)Lq * p.Dp * 2 * nqp, kb = (size_t)Lk * p.Dp * 2 * nqp, vb = (size_t)Lk * p.Dp * 2 * NV, sb = (size_t)nq * nk * F3_T * F3_T * 4, tb = (size_t)nq * F3_T * 4;
+    const size_t per_head = qb + kb + vb + sb + tb;
     long long G = (long long)(scratch_cap / per_head);
     if (G < 1) G = 1;
     if (G > BH) G = BH;
@@ -648,7 +692,7 @@ inline int f32tc_run(const b200attn_args &a, int rd, float base, F32Scratch &sc,
         if (cudaMemsetAsync(sc.mark, 0, 256, st) != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "cudaMemsetAsync failed"); return B200ATTN_ERR_CUDA; }
     }
     p.c = 1.4426950408889634f / sqrtf((float)D);
-    p.vec_out = D % 4 == 0 && ((uintptr_t)a.out & 15) == 0;
+    p.vec_out = D % 4 == 0 && ((uintptr_t)a.out & (4 * sizeof(T) - 1)) == 0;
     p.mark = sc.mark;
     p.err = err_dev; p.err_sys = err_sys; p.spin_limit = spin_limit;
     for (long long h0 = 0; h0 < BH; h0 += G) {
@@ -657,12 +701,12 @@ inline int f32tc_run(const b200attn_args &a, int rd, float base, F32Scratch &sc,
         unsigned char *b = (unsigned char *)sc.buf;
         __nv_bfloat16 *qpl = (__nv_bfloat16 *)b; b += up(n * qb);
         __nv_bfloat16 *kpl = (__nv_bfloat16 *)b; b += up(n * kb);
-        __nv_bfloat16 *vpl = (__nv_bfloat16 *)b; b += up(n * kb);
+        __nv_bfloat16 *vpl = (__nv_bfloat16 *)b; b += up(n * vb);
         p.S = (float *)b; b += up(n * sb);
         p.rowmax = (int *)b;
         p.q = qpl; p.k = kpl; p.v = vpl;
         p.heads = n;
-        p.O = (float *)a.out + (size_t)h0 * Lq * D;
+        p.O = (T *)a.out + (size_t)h0 * Lq * D;
         if (++sc.calls == 0) sc.calls = 1;
         p.call = sc.calls;
         F32SplitParams s{};
@@ -671,12 +715,12 @@ inline int f32tc_run(const b200attn_args &a, int rd, float base, F32Scratch &sc,
         s.cos_cache = a.cos_cache; s.sin_cache = a.sin_cache;
         s.mark = sc.mark; s.call = p.call;
         s.rowmax = p.rowmax; s.nrows = (long long)n * nq * F3_T;
-        s.t[0] = {(const float *)a.Q + (size_t)h0 * Lq * D, qpl, Lq, a.pe != B200ATTN_PE_NONE};
-        s.t[1] = {(const float *)a.K + (size_t)h0 * Lk * D, kpl, Lk, pe_encodes_k(a.pe)};
-        s.t[2] = {(const float *)a.V + (size_t)h0 * Lk * D, vpl, Lk, 0};
+        s.t[0] = {(const T *)a.Q + (size_t)h0 * Lq * D, qpl, Lq, a.pe != B200ATTN_PE_NONE, nqp, nqp > 1};
+        s.t[1] = {(const T *)a.K + (size_t)h0 * Lk * D, kpl, Lk, pe_encodes_k(a.pe), nqp, nqp > 1};
+        s.t[2] = {(const T *)a.V + (size_t)h0 * Lk * D, vpl, Lk, 0, NV, 1};
         CUtensorMap tmQ, tmK, tmV;
-        if (!make_tmap_grouped_heads(&tmQ, qpl, 3ll * n, Lq, p.Dp, F3_T, 1) || !make_tmap_grouped_heads(&tmK, kpl, 3ll * n, Lk, p.Dp, F3_T, 1) ||
-            !make_tmap_grouped_heads(&tmV, vpl, 3ll * n, Lk, p.Dp, 64, 1)) {
+        if (!make_tmap_grouped_heads(&tmQ, qpl, (long long)nqp * n, Lq, p.Dp, F3_T, 1) || !make_tmap_grouped_heads(&tmK, kpl, (long long)nqp * n, Lk, p.Dp, F3_T, 1) ||
+            !make_tmap_grouped_heads(&tmV, vpl, (long long)NV * n, Lk, p.Dp, 64, 1)) {
             snprintf(t_tc_error, sizeof t_tc_error, "cuTensorMapEncodeTiled failed");
             return h0 == 0 ? -1 : B200ATTN_ERR_CUDA;
         }
@@ -688,21 +732,28 @@ inline int f32tc_run(const b200attn_args &a, int rd, float base, F32Scratch &sc,
         shares = cap / blocks;
         if (shares > (n + 1) / 2) shares = (n + 1) / 2;
         if (shares < 1) shares = 1;
-        cudaError_t e = launch_dependent(f32_split_kernel, dim3((unsigned)blocks, (unsigned)shares, 3), 256, 0, 1, st, s);
+        cudaError_t e = launch_dependent(f32_split_kernel<T>, dim3((unsigned)blocks, (unsigned)shares, 3), 256, 0, 1, st, s);
         // scores: a CTA per SM, a tile at a time
         const long long tiles = nq * nk * n;
         const unsigned grid = (unsigned)(tiles < sm_count ? tiles : sm_count);
-        if (e == cudaSuccess) e = launch_dependent(f32_scores_kernel, dim3(grid), F3_A_THREADS, smem_a, 1, st, tmQ, tmK, p);
+        if (e == cudaSuccess) e = launch_dependent(nqp == 3 ? f32_scores_kernel<3> : f32_scores_kernel<NV>, dim3(grid), F3_A_THREADS, smem_a(nqp), 1, st, tmQ, tmK, p);
         // P V: the keys are cut while that still adds CTAs to idle SMs and leaves each a step for either set of warps
         const int nu = (Lk + 63) / 64;
         int ncl = 1;
         while (ncl < F3_MAX_CLUSTER && 4 * ncl <= nu && nq * ndb * n * ncl * 2 <= sm_count) ncl *= 2;
         p.upc = (nu + ncl - 1) / ncl;
-        if (e == cudaSuccess) e = launch_dependent(f32_pv_kernel, dim3((unsigned)ncl, (unsigned)(nq * ndb), (unsigned)n), F3_B_THREADS, smem_b, ncl, st, tmV, p);
+        if (e == cudaSuccess) e = launch_dependent(f32_pv_kernel<T, NV>, dim3((unsigned)ncl, (unsigned)(nq * ndb), (unsigned)n), F3_B_THREADS, smem_b, ncl, st, tmV, p);
         if (e != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "launch of the fp32 tensor-core kernels failed: %s", cudaGetErrorString(e)); return B200ATTN_ERR_CUDA; }
         launches->fetch_add(3);
     }
     return B200ATTN_OK;
+}
+
+inline int f32tc_run(const b200attn_args &a, int rd, float base, F32Scratch &sc, unsigned *err_dev, unsigned *err_sys, int sm_count, unsigned spin_limit,
+                     size_t scratch_cap, cudaStream_t st, std::atomic<unsigned long long> *launches) {
+    return a.dtype == B200ATTN_F32 ? f32tc_launch<float>(a, rd, base, sc, err_dev, err_sys, sm_count, spin_limit, scratch_cap, st, launches)
+         : a.dtype == B200ATTN_F16 ? f32tc_launch<__half>(a, rd, base, sc, err_dev, err_sys, sm_count, spin_limit, scratch_cap, st, launches)
+                                   : f32tc_launch<__nv_bfloat16>(a, rd, base, sc, err_dev, err_sys, sm_count, spin_limit, scratch_cap, st, launches);
 }
 
 }  // namespace b200attn

@@ -1,4 +1,4 @@
-// bf16 / fp16 attention forward for narrow heads (head_d up to 256) as ONE kernel on the 5th-generation tensor
+// bf16 / fp16 attention forward for narrow heads (head_d 64, 128, 192 or 256) as ONE kernel on the 5th-generation tensor
 // cores: the scores never leave the SM.  (At these widths the two-kernel path of tc_wide.cuh is bound by the
 // HBM round trip of its score scratch, whose bytes per FLOP grow as 1 / head_d.)  Same mathematics as the
 // reference's bf16 forward, kernels/attention_bf16_optimized_fused.cu:493-505: softmax(Q K^T / sqrt(d)) V with
@@ -9,14 +9,10 @@
 // MMAs; warpgroups of 128 threads - a thread per query row, which is a lane of tensor memory - do the online
 // softmax and, at the end of a unit, the epilogue O / row sum -> 16 bit -> global.  Score tiles and output
 // accumulators live in tensor memory (512 columns: the budget that shapes both layouts).
-//   fa_kernel     head_d <= 128: units of (head, 256 query rows) = two query tiles, P through shared memory;
-//   fa256_kernel  head_d 136 to 256: units of (head, 128 query rows), two score buffers, P through tensor memory.
-// head_d is any multiple of 8 (16-byte rows: what a tensor map can describe).  Tiles keep whole 64-column groups in shared
-// memory; the MMAs take ceil(head_d / 16) steps of the score contraction and as many 16-column pieces of the output, so a
-// width between the group sizes costs its own arithmetic.  A width that is not a multiple of 64 is loaded a group per
-// request, columns beyond head_d reading as zero (a multiple of 64: one request per tile).  Such widths used to run on
-// the CUDA-core kernels of splitd.cuh: 2 x 16 heads, 777 x 1000, head_d 96, bf16: 720 -> 25 us; 1 x 32 heads, 4 x 8192, head_d
-// 96: 748 -> 100 us; head_d 192 (2 x 16, 777 x 1000) on the two-kernel path of tc_wide.cuh: 56 -> 39 us.
+//   fa_kernel     head_d 64 / 128: units of (head, 256 query rows) = two query tiles, P through shared memory;
+//   fa256_kernel  head_d 192 / 256: units of (head, 128 query rows), two score buffers, P through tensor memory.
+// Other widths keep probabilities and encoded operands in fp32 (tc_f32.cuh): a step to any multiple of 8 here rounded both to 16
+// bits where no 16-bit kernel had been.  head_d 192 (2 x 16 heads, 777 x 1000, bf16) 39 us, on the two-kernel path of tc_wide.cuh 56 us.
 // The ring position (stage, parity) of the loading and issuing threads is kept incrementally: a division by the
 // run-time stage count cost such a thread some 400 clocks per wait and, at head_d 256, a sixth of the throughput.
 //
@@ -37,8 +33,6 @@ constexpr float FA_RESCALE_LOG2 = 8.0f;   // the accumulator is rescaled when a 
 
 struct FaParams {
     int Lq, Lk, D;
-    int ks;                    // ceil(D / 16): MMA steps of the score contraction, 16-column pieces of the output
-    int grouped;               // D % 64 == 0: the maps hold the 64-column groups as a coordinate, one request per tile
     int nqp;                   // pairs of query tiles per head: ceil(ceil(Lq / 128) / 2)
     int nkt;                   // key tiles: ceil(Lk / 128)
     int nst;                   // ring stages (fa_kernel: [128 keys x head_d] each; fa256_kernel: 32 KB each)
@@ -114,15 +108,8 @@ constexpr int FA_THREADS = 384;      // warpgroup 0: warp 0 loads, warps 1 and 2
 constexpr int FA_REGS_SMALL = 80, FA_REGS_LARGE = 208;   // registers per thread after the hand-over: 128 * 80 + 256 * 208 <= 384 * 168
 constexpr uint32_t FA_P_BYTES = 128u * 128u * 2u;   // a P tile: [2 groups of 64 keys][128 rows][128 B]
 
-// rows [row, row + box rows) of a head, column groups [g0, g0 + n), as consecutive [rows][128 B] slabs at `dst`
-__device__ __forceinline__ void fa_load_tile(unsigned char *dst, const CUtensorMap *tm, const FaParams &p, int row, int bh, int g0, int n, int slab_bytes, uint64_t *bar) {
-    if (p.grouped) tma_load_4d(dst, tm, 0, row, g0, bh, bar);
-    else for (int g = 0; g < n; ++g) tma_load_3d(dst + (size_t)g * slab_bytes, tm, (g0 + g) * 64, row, bh, bar);
-}
-
-// Epilogue of one accumulator row [head_d] by the row's thread: O / row sum -> 16 bit -> global.  Whole 64-column groups:
-// lanes trade pieces so that the stores cover full lines; what is left (or rows that are not 32-byte aligned): the thread's
-// own pieces of 16 bytes.  `orow` = the row's place in the output, `left` = rows of the head from this one's group of four on.
+// Epilogue of one accumulator row [head_d] by the row's thread: O / row sum -> 16 bit -> global.  Lanes
+// trade pieces so that the stores cover full lines.  `orow` = the row's place in the output, `left` = rows of the head from this one's group of four on.
 template <bool F16>
 __device__ __forceinline__ void fa_store_row(uint32_t to, float inv, __nv_bfloat16 *orow, int D, int lane, int left, uint32_t (&r0)[32], uint32_t (&r1)[32]) {
     for (int c0 = 0; c0 < D; c0 += 64) {
@@ -133,13 +120,7 @@ __device__ __forceinline__ void fa_store_row(uint32_t to, float inv, __nv_bfloat
 #pragma unroll
             for (int i = 0; i < 16; ++i) r1[16 * hh + i] = pack_16x2(__uint_as_float(r0[2 * i]) * inv, __uint_as_float(r0[2 * i + 1]) * inv, F16);
         }
-        if (c0 + 64 <= D && (D & 15) == 0) {
-            store_rows_128B_transposed_if(reinterpret_cast<unsigned char *>(orow - (long long)(lane & 3) * D + c0), (size_t)D * 2, r1, lane, left);
-        } else if ((lane & 3) < left) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (c0 + 8 * i < D) *reinterpret_cast<uint4 *>(orow + c0 + 8 * i) = make_uint4(r1[4 * i], r1[4 * i + 1], r1[4 * i + 2], r1[4 * i + 3]);
-        }
+        store_rows_128B_transposed_if(reinterpret_cast<unsigned char *>(orow - (long long)(lane & 3) * D + c0), (size_t)D * 2, r1, lane, left);
     }
 }
 
@@ -156,9 +137,9 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
     const uint32_t raw_addr = smem_u32(fa_smem_raw);
     unsigned char *smem = fa_smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int D = p.D, nkt = p.nkt, nst = p.nst, ks = p.ks;
-    const int ng = (D + 63) >> 6;
-    const uint32_t tile_bytes = (uint32_t)FA_BN * 128u * (uint32_t)ng;   // a Q, K or V tile: [ng groups][128 rows][128 B]
+    const int D = p.D, nkt = p.nkt, nst = p.nst;
+    const int ng = D >> 6;
+    const uint32_t tile_bytes = (uint32_t)FA_BN * (uint32_t)D * 2u;   // a Q, K or V tile: [ng groups][128 rows][128 B]
     unsigned char *q_smem = smem;                                      // two Q tiles
     unsigned char *p_smem = smem + 2 * (size_t)tile_bytes;             // two P tiles
     unsigned char *ring = p_smem + 2 * (size_t)FA_P_BYTES;
@@ -206,7 +187,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
                 TC_PROF(0);
                 if (!ok) return;
                 mbar_expect_tx(&bars.kv_full[s], tile_bytes);
-                fa_load_tile(ring + (size_t)s * tile_bytes, tm, p, j * FA_BN, bh, 0, ng, FA_BN * 128, &bars.kv_full[s]);
+                tma_load_4d(ring + (size_t)s * tile_bytes, tm, 0, j * FA_BN, 0, bh, &bars.kv_full[s]);
                 if (++s == nst) { s = 0; ph ^= 1u; }
             };
             for (long long unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x, ++ui) {
@@ -214,7 +195,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
                 ok = mbar_wait(&bars.q_empty, (uint32_t)(ui & 1) ^ 1u, lim);
                 if (!ok) break;
                 mbar_expect_tx(&bars.q_full, 2 * tile_bytes);
-                for (int t = 0; t < 2; ++t) fa_load_tile(q_smem + t * tile_bytes, &tmQ, p, (qp * 2 + t) * FA_BM, bh, 0, ng, FA_BM * 128, &bars.q_full);
+                for (int t = 0; t < 2; ++t) tma_load_4d(q_smem + t * tile_bytes, &tmQ, 0, (qp * 2 + t) * FA_BM, 0, bh, &bars.q_full);
                 load_kv(&tmK, bh, 0);                     // the order of the issuers: K_0 | K_1, V_0 | K_2, V_1 | ...
                 for (int j = 0; j < nkt && ok; ++j) {
                     if (j + 1 < nkt) load_kv(&tmK, bh, j + 1);
@@ -227,7 +208,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
       } else if (warp < 3) {
         if (elect_one()) {
             const int t = warp - 1;
-            const uint32_t id_qk = umma_idesc_16(FA_BM, FA_BN, 0, 0, F16 ? 1 : 0), id_pv = umma_idesc_16(FA_BM, 16 * ks, 0, 1, F16 ? 1 : 0);
+            const uint32_t id_qk = umma_idesc_16(FA_BM, FA_BN, 0, 0, F16 ? 1 : 0), id_pv = umma_idesc_16(FA_BM, D, 0, 1, F16 ? 1 : 0);
             const uint32_t qa = smem_u32(q_smem + (size_t)t * tile_bytes), pa = smem_u32(p_smem + (size_t)t * FA_P_BYTES);
             const uint32_t t_s = tmem + t * 128, t_o = tmem + 256 + t * 128;
             int s = 0;             // ring stage and the parity of its use
@@ -245,8 +226,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
                 for (int g = 0; g < ng; ++g) {
                     const uint64_t dq = umma_desc_k_sw128(qa + g * (FA_BM * 128)), dk = umma_desc_k_sw128(ka + g * (FA_BN * 128));
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (4 * g + k < ks) umma_bf16(t_s, dq + 2 * k, dk + 2 * k, id_qk, (g | k) != 0);
+                    for (int k = 0; k < 4; ++k) umma_bf16(t_s, dq + 2 * k, dk + 2 * k, id_qk, (g | k) != 0);
                 }
                 umma_commit(&bars.s_full[t]);
                 umma_commit(&bars.kv_empty[s]);
@@ -368,7 +348,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
                         const float m_new = need ? mx : m_ref;
                         const float f = fast_exp2(m_ref - m_new);
                         uint32_t w[16];
-                        for (int c = 0; c < ks; ++c) {
+                        for (int c = 0; c < (D >> 4); ++c) {
                             tmem_ld16(to + 16 * c, w);
                             tmem_ld_wait();
 #pragma unroll
@@ -437,7 +417,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUten
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 // ---------------------------------------------------------------------------------------------------
-// head_d 136 to 256: ONE query tile of 128 rows per unit.  The output accumulator [128 x 256] fp32 takes half of the tensor
+// head_d 192 / 256: ONE query tile of 128 rows per unit.  The output accumulator [128 x 256] fp32 takes half of the tensor
 // memory; the other half holds two score buffers, so that S_j+1 = Q K_j+1^T is computed while the softmax warps work
 // on S_j.  P (16 bit) is written over the first 64 columns of its own score buffer and the P V MMA takes its A operand
 // from tensor memory (umma_16_ts), so P never touches shared memory:   S_0 | S_1, O += P_0 V_0, S_2, O += P_1 V_1, S_3, ...   K and V pass through the ring
@@ -457,9 +437,8 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     const uint32_t raw_addr = smem_u32(fa_smem_raw);
     unsigned char *smem = fa_smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nkt = p.nkt, nst = p.nst, ks = p.ks;
-    const int ng = (p.D + 63) >> 6;                     // 3 or 4
-    unsigned char *q_smem = smem;                       // [ng groups][128 rows][128 B]
+    const int nkt = p.nkt, nst = p.nst, ks = p.D >> 4;  // MMA steps of the score contraction
+    unsigned char *q_smem = smem;                       // [4 groups][128 rows][128 B], groups beyond head_d are zero
     unsigned char *ring = smem + 2 * FB_STAGE;
     const uint32_t lim = p.spin_limit;
 
@@ -492,9 +471,8 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
                 for (int h = 0; h < 2 && ok; ++h) {
                     ok = mbar_wait(&bars.kv_empty[s], ph ^ 1u, lim);
                     if (!ok) break;
-                    const int n = min(2, ng - 2 * h);
-                    mbar_expect_tx(&bars.kv_full[s], p.grouped ? FB_STAGE : n * FA_BN * 128);   // (a grouped box is whole, groups beyond head_d read as zero)
-                    fa_load_tile(ring + (size_t)s * FB_STAGE, &tmK, p, j * FA_BN, bh, 2 * h, n, FA_BN * 128, &bars.kv_full[s]);
+                    mbar_expect_tx(&bars.kv_full[s], FB_STAGE);
+                    tma_load_4d(ring + (size_t)s * FB_STAGE, &tmK, 0, j * FA_BN, 2 * h, bh, &bars.kv_full[s]);
                     if (++s == nst) { s = 0; ph ^= 1u; }
                 }
             };
@@ -502,8 +480,8 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
                 for (int h = 0; h < 2 && ok; ++h) {
                     ok = mbar_wait(&bars.kv_empty[s], ph ^ 1u, lim);
                     if (!ok) break;
-                    mbar_expect_tx(&bars.kv_full[s], p.grouped ? FB_STAGE : ng * 64 * 128);
-                    fa_load_tile(ring + (size_t)s * FB_STAGE, &tmV, p, j * FA_BN + 64 * h, bh, 0, ng, 64 * 128, &bars.kv_full[s]);
+                    mbar_expect_tx(&bars.kv_full[s], FB_STAGE);
+                    tma_load_4d(ring + (size_t)s * FB_STAGE, &tmV, 0, j * FA_BN + 64 * h, 0, bh, &bars.kv_full[s]);
                     if (++s == nst) { s = 0; ph ^= 1u; }
                 }
             };
@@ -512,8 +490,8 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
                 const int bh = (int)(unit / p.nqp), qt = (int)(unit % p.nqp);
                 ok = mbar_wait(&bars.q_empty, (uint32_t)(ui & 1) ^ 1u, lim);
                 if (!ok) break;
-                mbar_expect_tx(&bars.q_full, p.grouped ? 2 * FB_STAGE : ng * FA_BM * 128);
-                fa_load_tile(q_smem, &tmQ, p, qt * FA_BM, bh, 0, ng, FA_BM * 128, &bars.q_full);
+                mbar_expect_tx(&bars.q_full, 2 * FB_STAGE);
+                tma_load_4d(q_smem, &tmQ, 0, qt * FA_BM, 0, bh, &bars.q_full);
                 load_k(bh, 0, ok);                        // the order of the MMA thread: K_0 | K_1, V_0, K_2, V_1, ...
                 for (int j = 0; j < nkt && ok; ++j) {
                     if (j + 1 < nkt) load_k(bh, j + 1, ok);
@@ -524,7 +502,7 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
         }
     } else if (warp == 1) {
         if (elect_one()) {
-            const uint32_t id_qk = umma_idesc_16(FA_BM, FA_BN, 0, 0, F16 ? 1 : 0), id_pv = umma_idesc_16(FA_BM, 16 * ks, 0, 1, F16 ? 1 : 0);
+            const uint32_t id_qk = umma_idesc_16(FA_BM, FA_BN, 0, 0, F16 ? 1 : 0), id_pv = umma_idesc_16(FA_BM, p.D, 0, 1, F16 ? 1 : 0);
             int s = 0;                  // ring stage and the parity of its use
             uint32_t ph = 0;
             long long gt = 0;           // tiles issued so far (score buffer = tile & 1)
@@ -717,10 +695,10 @@ fa256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
 // ---- host side ------------------------------------------------------------------------------------
 inline bool fa_supported(const b200attn_args &a) {
     if (a.dtype != B200ATTN_BF16 && a.dtype != B200ATTN_F16) return false;
-    if (a.head_d % 8 != 0 || a.head_d > FB_D) return false;
-    // few queries: the key-split kernels, or the split-head_d kernels; at the widths those do not take on the tensor cores
-    // a CTA per head here still beats the CUDA-core kernels once the keys fill more than half a tile
-    if (a.len_q <= 64 && (a.len_k <= 64 || a.head_d % 64 == 0)) return false;
+    if (a.head_d % 64 != 0 || a.head_d > FB_D) return false;
+    // head_d 192: what the two-kernel path takes, with the same roundings; its bf16 encodings and longer keys stay in fp32 (tc_f32.cuh)
+    if (a.head_d == 192 && ((a.dtype == B200ATTN_BF16 && a.pe != B200ATTN_PE_NONE) || a.len_k > 65536)) return false;
+    if (a.len_q <= 64) return false;   // few queries: the key-split kernels, or the split-head_d kernels
     if ((((uintptr_t)a.Q | (uintptr_t)a.K | (uintptr_t)a.V) & 15) != 0 || ((uintptr_t)a.out & 31) != 0) return false;
     const long long BH = (long long)a.batch_sz * a.num_heads;
     if (BH >= (1ll << 31) || BH * ((a.len_q + 255) / 256) >= (1ll << 40)) return false;
@@ -755,24 +733,19 @@ inline int fa_run(const b200attn_args &a, unsigned *err_dev, unsigned *err_sys, 
             smem_max[dev & 63] = (size_t)dyn;
         }
     }
-    const bool grouped = D % 64 == 0;
-    const int ng = (D + 63) / 64;
-    // the map of one operand: box of `box_rows` rows and `box_groups` 64-column groups, or of one group where a row is not whole groups
-    auto make_map = [&](CUtensorMap *m, const void *base, int rows, int box_rows, int box_groups) {
-        return grouped ? make_tmap_grouped_heads(m, base, BH, rows, D, box_rows, box_groups) : make_tmap_cols_heads(m, base, BH, rows, D, box_rows);
-    };
     if (D > 128) {
         // one query tile per unit, K and V through the ring in halves
         int nst = (int)((smem_max[dev & 63] - 1024 - 2 * FB_STAGE) / FB_STAGE);
         if (nst > FA_MAX_STAGES) nst = FA_MAX_STAGES;
         if (nst < 5) return -1;
         CUtensorMap tmQ, tmK, tmV;
-        if (!make_map(&tmQ, a.Q, Lq, FA_BM, 4) || !make_map(&tmK, a.K, Lk, FA_BN, 2) || !make_map(&tmV, a.V, Lk, 64, 4)) {
+        if (!make_tmap_grouped_heads(&tmQ, a.Q, BH, Lq, D, FA_BM, 4) || !make_tmap_grouped_heads(&tmK, a.K, BH, Lk, D, FA_BN, 2) ||
+            !make_tmap_grouped_heads(&tmV, a.V, BH, Lk, D, 64, 4)) {
             snprintf(t_tc_error, sizeof t_tc_error, "cuTensorMapEncodeTiled failed");
             return -1;
         }
         FaParams p{};
-        p.Lq = Lq; p.Lk = Lk; p.D = D; p.ks = (D + 15) / 16; p.grouped = grouped ? 1 : 0;
+        p.Lq = Lq; p.Lk = Lk; p.D = D;
         p.nqp = (Lq + FA_BM - 1) / FA_BM;   // query tiles per head
         p.nkt = (Lk + FA_BN - 1) / FA_BN;
         p.nst = nst;
@@ -790,17 +763,18 @@ inline int fa_run(const b200attn_args &a, unsigned *err_dev, unsigned *err_sys, 
         launches->fetch_add(1);
         return B200ATTN_OK;
     }
-    const size_t tb = (size_t)FA_BN * 128 * ng;
+    const size_t tb = (size_t)FA_BN * D * 2;
     int nst = (int)((smem_max[dev & 63] - 1024 - 2 * tb - 2 * (size_t)FA_P_BYTES) / tb);   // head_d 128: 3 stages; 64: 8
     if (nst > FA_MAX_STAGES) nst = FA_MAX_STAGES;
     if (nst < 3) return -1;
     CUtensorMap tmQ, tmK, tmV;
-    if (!make_map(&tmQ, a.Q, Lq, FA_BM, ng) || !make_map(&tmK, a.K, Lk, FA_BN, ng) || !make_map(&tmV, a.V, Lk, FA_BN, ng)) {
+    if (!make_tmap_grouped_heads(&tmQ, a.Q, BH, Lq, D, FA_BM, D / 64) || !make_tmap_grouped_heads(&tmK, a.K, BH, Lk, D, FA_BN, D / 64) ||
+        !make_tmap_grouped_heads(&tmV, a.V, BH, Lk, D, FA_BN, D / 64)) {
         snprintf(t_tc_error, sizeof t_tc_error, "cuTensorMapEncodeTiled failed");
         return -1;
     }
     FaParams p{};
-    p.Lq = Lq; p.Lk = Lk; p.D = D; p.ks = (D + 15) / 16; p.grouped = grouped ? 1 : 0;
+    p.Lq = Lq; p.Lk = Lk; p.D = D;
     p.nqp = ((Lq + FA_BM - 1) / FA_BM + 1) / 2;
     p.nkt = (Lk + FA_BN - 1) / FA_BN;
     p.nst = nst;

@@ -1,4 +1,4 @@
-"""GPU parity of the one-kernel tensor-core path for narrow heads (head_d 64, 128 or 256, bf16 / fp16,
+"""GPU parity of the one-kernel tensor-core path for narrow heads (head_d 64, 128, 192 or 256, bf16 / fp16,
 more than 64 queries): scores and the output accumulator stay in tensor memory, online softmax with a lazily
 rescaled accumulator.  Oracle: fp32 CPU attention on the 16-bit-rounded inputs; tolerance max-abs 2e-2 (bf16)."""
 import numpy as np
@@ -211,22 +211,47 @@ def test_fused_path_very_long_keys(pkg, cuda):
 @pytest.mark.parametrize("D", [8, 40, 72, 80, 96, 104, 136, 160, 192, 200, 248])
 @pytest.mark.parametrize("lens", [(130, 300), (300, 129), (3, 200)], ids=str)
 def test_widths_between_the_column_groups(pkg, cuda, D, lens):
-    """Any multiple of 8: widths whose last 16-column step is half empty (8, 40, 72, 104, ...), whose last 64-column group is
-    short, and a whole number of groups that is not a power of two (192); a few queries too where no other tensor-core
-    path takes the width.  Nothing behind the output is written."""
+    """Any multiple of 8 below 256: the operands are exact, encoded operands, scores, probabilities and sums fp32, and only the
+    result is rounded to 16 bits (head_d 192 without an encoding: P rounded too, as at 64, 128 and 256).  Nothing behind the
+    output is written."""
     import torch
     (Lq, Lk), B, H = lens, 1, 3
     bits, up = bf16_problem(B, H, Lq, Lk, D, 100 + D, "normal")
-    want = ol.attention(*up)
     q, k, v = (bf16_to_dev(b, cuda) for b in bits)
-    big = torch.full((B * H * Lq * D + 256,), 3.0, dtype=torch.bfloat16, device=cuda)
-    out = big[:B * H * Lq * D].view(B, H, Lq, D)
-    pkg.forward(q, k, v, out=out)
-    assert pkg.last_path() == ("tc_wide" if D == 192 and Lq <= 64 else "tc_fused"), pkg.last_path()
-    assert bool((big[B * H * Lq * D:] == 3.0).all())
-    assert float(np.abs(bf16_from_dev(out) - want).max()) <= 8e-3   # the bound of the whole widths: P and the result rounded to bf16
-    got = pkg.forward(*(t.to(torch.float16) for t in (q, k, v)))
-    assert float(np.abs(got.float().cpu().numpy() - want).max()) <= 4e-3   # fp16: the suite's bound
-    if D % 16 == 0:
-        got = run(pkg, cuda, bits, pe=pkg.PE_ROPE_INTERLEAVED)
-        assert float(np.abs(got - ol.attention(*up, pe=ol.PE_ROPE_INTERLEAVED)).max()) <= TOL
+    path = ("tc_wide" if Lq <= 64 else "tc_fused") if D == 192 else "tc_f32"
+    for dtype, half_ulp in ((torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)):   # relative, at most
+        tq, tk, tv = (t.to(dtype) for t in (q, k, v))
+        big = torch.full((B * H * Lq * D + 256,), 3.0, dtype=dtype, device=cuda)
+        out = big[:B * H * Lq * D].view(B, H, Lq, D)
+        for pe in (pkg.PE_NONE, pkg.PE_ROPE_INTERLEAVED, pkg.PE_ROPE_HALF, pkg.PE_SINUSOIDAL):
+            if D == 192 and pe != pkg.PE_NONE and (Lq <= 64 or dtype == torch.float16):
+                continue   # other kernels, other tests
+            pkg.forward(tq, tk, tv, out=out, pe=pe)
+            assert pkg.last_path() == ("tc_f32" if pe != pkg.PE_NONE else path), (pkg.last_path(), pe)
+            assert bool((big[B * H * Lq * D:] == 3.0).all())
+            want = ol.attention(*(t.float().cpu().numpy() for t in (tq, tk, tv)), pe=pe)
+            err = np.abs(out.float().cpu().numpy() - want)
+            if pkg.last_path() == "tc_f32":
+                # half a unit in the last place of the result, and fp32: sums to 1e-5, angles up to 300 and their functions to a few
+                # ulp, which enter a score of normal values (up to 16 or so) with the weights of head_d / 2 pairs
+                assert (err <= np.abs(want) * half_ulp + (1e-5 if pe == pkg.PE_NONE else 1e-3)).all(), (dtype, pe, err.max())
+            else:
+                assert err.max() <= (8e-3 if dtype == torch.bfloat16 else 4e-3), (dtype, pe, err.max())   # the bounds of the whole widths
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("f16", [False, True])
+@pytest.mark.parametrize("pe", ["none", "rope"])
+def test_non_finite_values_at_other_widths(pkg, cuda, which, value, f16, pe):
+    """As on the CUDA cores, which took these widths before (a key or row that is not finite, not only an element)."""
+    import torch
+    dtype, kind = torch.float16 if f16 else torch.bfloat16, pkg.PE_NONE if pe == "none" else pkg.PE_ROPE_INTERLEAVED
+    T = [torch.randn(1, 2, 150, 72, generator=torch.Generator().manual_seed(5 + i)).to(dtype).to(cuda) for i in range(3)]
+    T[which][0, 1, 7, 5] = value
+    T[which][0, 0, 140] = value
+    got = pkg.forward(*T, pe=kind)
+    assert pkg.last_path() == "tc_f32"
+    want = pkg.forward(*T, pe=kind, flags=pkg.FLAG_FORCE_GENERIC)
+    assert pkg.last_path() == "splitd_two_pass"
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
