@@ -409,7 +409,11 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                             for (int i = 0; i < NVP; ++i) *reinterpret_cast<uint4 *>(d + i * 2 * SW_PL) = w[i];
                         }
                     }
-                    if (odd != odd) *reinterpret_cast<volatile unsigned *>(&s_odd_v[e]) = (unsigned)b + 1u;
+                    if (__any_sync(0xffffffffu, odd != odd)) {
+                        // the word still belongs to block b - 2 until its epilogue, which may be in plain loops, has read it
+                        SW_WARP_WAIT(11, bars.o_empty[e], ((b >> 1) & 1) ^ 1);
+                        if (lane == 0) *reinterpret_cast<volatile unsigned *>(&s_odd_v[e]) = (unsigned)b + 1u;
+                    }
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) { mbar_arrive(&bars.v_ready[e]); mbar_arrive(&bars.v_free[s]); }

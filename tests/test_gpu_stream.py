@@ -96,6 +96,22 @@ def test_non_finite_values_as_on_the_cuda_cores(pkg, cuda, dtype, which, value):
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,D,L", [(148, 512, 64), (148, 640, 33), (20, 4096, 64)])
+def test_non_finite_values_in_many_blocks(pkg, cuda, dtype, H, D, L):
+    """A key whose whole V row is infinite, in slices of four and more blocks of output columns: the plain loops of one block's
+    epilogue are still running when blocks further on have been split and multiplied."""
+    T = [to_dev(x, cuda).to(dtype) for x in ol.make_qkv(1, H, L, L, D, 94, "uniform")]
+    T[2][0, :, 5] = float("inf")
+    T[2][0, 3, 9, ::2] = float("-inf")
+    want = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED, flags=pkg.FLAG_FORCE_GENERIC)
+    assert pkg.last_path().startswith("splitd_") and pkg.last_path() != "splitd_stream"
+    for _ in range(3):
+        got = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED)
+        assert pkg.last_path() == "splitd_stream"
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isposinf(got), torch.isposinf(want)) and torch.equal(torch.isneginf(got), torch.isneginf(want))
+
+
 @pytest.mark.parametrize("pe", [ol.PE_NONE, ol.PE_SINUSOIDAL])
 @pytest.mark.parametrize("H,Lq,Lk,D,n", [(4, 64, 64, 512, 5), (1, 16, 64, 64, 17), (30, 33, 20, 1000, 6), (148, 8, 8, 64, 2)])
 def test_one_launch_for_several_problems(pkg, cuda, pe, H, Lq, Lk, D, n):
