@@ -443,7 +443,11 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                     if (NQP > 1) { tmem_ld16(ts + 64 + 16 * k, r1); tmem_ld16(ts + 128 + 16 * k, r2); }
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[16 * k + j] += NQP > 1 ? __uint_as_float(r0[j]) + (__uint_as_float(r1[j]) + __uint_as_float(r2[j])) : __uint_as_float(r0[j]);
+                    for (int j = 0; j < 16; ++j) {
+                        // (products that overflow: the smaller ones may be infinities of the other sign, a third piece need not have its value's)
+                        const float lead = __uint_as_float(r0[j]);
+                        acc[16 * k + j] += NQP > 1 && fabsf(lead) < INFINITY ? lead + (__uint_as_float(r1[j]) + __uint_as_float(r2[j])) : lead;
+                    }
                 }
                 tc_fence_before();
                 __syncwarp();

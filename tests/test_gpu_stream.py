@@ -112,6 +112,24 @@ def test_non_finite_values_in_many_blocks(pkg, cuda, dtype, H, D, L):
         assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isposinf(got), torch.isposinf(want)) and torch.equal(torch.isneginf(got), torch.isneginf(want))
 
 
+@pytest.mark.parametrize("dtype,pe,H,D", [(torch.float32, ol.PE_NONE, 148, 512), (torch.float32, ol.PE_ROPE_INTERLEAVED, 3, 304),
+                                           (torch.float32, ol.PE_ROPE_Q_ONLY, 148, 512), (torch.bfloat16, ol.PE_ROPE_INTERLEAVED, 3, 304)])
+def test_keys_of_minus_infinity_scores_have_no_weight(pkg, cuda, dtype, pe, H, D):
+    """Finite inputs whose products overflow: such keys have weight 0 and leave the others alone, as on the CUDA cores.  (1e30 =
+    9.95e29 + 4.70e27 - 4.08e24: the products with a third piece have the other sign.)  The last pair of columns: its angles
+    stay near 0, so that the rotation keeps the signs."""
+    T = [to_dev(x, cuda).to(dtype) for x in ol.make_qkv(1, H, 48, 60, D, 95, "uniform")]
+    T[0][..., -2], T[0][..., -1] = 1e30, 0.0
+    T[1][..., -2:] = 0.0
+    T[1][..., 20:40, -2] = -1e30
+    got = pkg.forward(*T, pe=pe)
+    assert pkg.last_path() == "splitd_stream"
+    want = pkg.forward(*T, pe=pe, flags=pkg.FLAG_FORCE_GENERIC)
+    assert torch.isfinite(want).all()
+    # (fp32: 1e-7 each; bf16: both round results that close once)
+    torch.testing.assert_close(got, want, rtol=1e-5 if dtype == torch.float32 else 2.0 ** -7, atol=MAX_ABS)
+
+
 @pytest.mark.parametrize("pe", [ol.PE_NONE, ol.PE_SINUSOIDAL])
 @pytest.mark.parametrize("H,Lq,Lk,D,n", [(4, 64, 64, 512, 5), (1, 16, 64, 64, 17), (30, 33, 20, 1000, 6), (148, 8, 8, 64, 2)])
 def test_one_launch_for_several_problems(pkg, cuda, pe, H, Lq, Lk, D, n):
