@@ -113,6 +113,8 @@ struct DeviceCtx {
     unsigned sdtc_gen_expect[ST_NBUF] = {};   // heads the earlier users of each buffer will have cleared
     bool sdtc_attr = false;
     bool sw_attr = false;
+    float *sw_S = nullptr;         // score scratch of the streamed split-head_d kernel: a head per SM
+    unsigned *sw_cnt = nullptr;
     SwTables sw_tables;            // angles of the streamed split-head_d kernel
     size_t sdtc_smem_max = 0;
     // the last enqueued call, when it was this kernel: a following call that is declared independent of it
@@ -196,6 +198,10 @@ static int ensure_scratch(DeviceCtx &c, size_t s_bytes, size_t n_counters, cudaS
             CU_TRY(cudaMemsetAsync(c.sdtc_cnt, 0, (size_t)ST_NBUF * c.sdtc_cap * 2 * sizeof(unsigned), st));
             CU_TRY(cudaMemsetAsync(c.sdtc_gen, 0, ST_NBUF * sizeof(unsigned), st));
             for (int i = 0; i < ST_NBUF; ++i) c.sdtc_gen_expect[i] = 0;
+        }
+        if (c.sw_S) {
+            CU_TRY(cudaMemsetAsync(c.sw_S, 0, (size_t)c.sm_count * 4096 * sizeof(float), st));
+            CU_TRY(cudaMemsetAsync(c.sw_cnt, 0, (size_t)c.sm_count * 2 * sizeof(unsigned), st));
         }
         CU_TRY(cudaMemsetAsync(c.err_dev, 0, sizeof(unsigned), st));
         c.scratch_dirty = false;
@@ -360,7 +366,7 @@ static int run_splitd(DeviceCtx &c, const b200attn_args &a, int rd, float base, 
     return B200ATTN_OK;
 }
 
-// the score-scratch ring of the tensor-core split-head_d kernels
+// the score-scratch ring of splitd_tc.cuh
 static int ensure_ring(DeviceCtx &c, cudaStream_t st) {
     if (c.sdtc_S == nullptr) {
         const int cap = c.sm_count;
@@ -538,6 +544,20 @@ static int launch_sw(DeviceCtx &c, const b200attn_args *a, int n, const SwParams
     return B200ATTN_OK;
 }
 
+// the score scratch of splitd_stream.cuh
+static int ensure_sw_scratch(DeviceCtx &c, cudaStream_t st) {
+    if (c.sw_S == nullptr) {
+        float *S = nullptr;
+        unsigned *cnt = nullptr;
+        CU_TRY(cudaMalloc(&S, (size_t)c.sm_count * 4096 * sizeof(float)));
+        cudaError_t e = cudaMalloc(&cnt, (size_t)c.sm_count * 2 * sizeof(unsigned));
+        if (e != cudaSuccess) { cudaFree(S); CU_TRY(e); }
+        c.sw_S = S; c.sw_cnt = cnt;
+        c.scratch_dirty = true;   // cleared below, on this call's stream
+    }
+    return c.scratch_dirty ? ensure_scratch(c, 0, 0, st) : B200ATTN_OK;
+}
+
 // One launch for `n` (<= SW_MAXP) problems of the same form, n heads' worth of CTAs on the chip at once.  -1: not taken, nothing launched.
 static int run_sw(DeviceCtx &c, const b200attn_args *a, int n, int rd, float base, cudaStream_t st) {
     const long long BH = (long long)a->batch_sz * a->num_heads, heads = n * BH;
@@ -549,14 +569,12 @@ static int run_sw(DeviceCtx &c, const b200attn_args *a, int n, int rd, float bas
         for (const void *k : kerns) CU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM));
         c.sw_attr = true;
     }
-    if (int rc = ensure_ring(c, st)) return rc;
+    if (int rc = ensure_sw_scratch(c, st)) return rc;
     SwParams p{};
     p.BH = (int)BH; p.Lq = a->len_q; p.Lk = a->len_k; p.D = a->head_d;
     p.natoms = (p.D + ST_ATOM - 1) / ST_ATOM;
     const int slots = (int)(c.sm_count / heads), per = (p.natoms + slots - 1) / slots;
     p.nsplit = (p.natoms + per - 1) / per;
-    const int buf = (int)(c.sdtc_seq % ST_NBUF);
-    p.buf = buf; p.cap_bh = c.sdtc_cap; p.gen_expect = c.sdtc_gen_expect[buf];
     p.pe = a->pe; p.rd = rd;
     if (a->pe != B200ATTN_PE_NONE) {
         const bool sinus = a->pe == B200ATTN_PE_SINUSOIDAL;
@@ -564,7 +582,7 @@ static int run_sw(DeviceCtx &c, const b200attn_args *a, int n, int rd, float bas
         if (p.tab == nullptr) return -1;
     }
     p.scale = 1.0f / sqrtf((float)p.D);
-    p.S = c.sdtc_S; p.counters = c.sdtc_cnt; p.gen = c.sdtc_gen;
+    p.S = c.sw_S; p.counters = c.sw_cnt;
     p.err = c.err_dev; p.err_sys = c.err_host_dev;
     p.spin_limit = current_spin_limit();
     p.wait_extra = g_test_wait_extra.load();
@@ -576,8 +594,6 @@ static int run_sw(DeviceCtx &c, const b200attn_args *a, int n, int rd, float bas
     else if (a->dtype == B200ATTN_F16) rc = pe ? launch_sw<__half, true, 1>(c, a, 1, p, st) : launch_sw<__half, false, 1>(c, a, 1, p, st);
     else rc = pe ? launch_sw<__nv_bfloat16, true, 1>(c, a, 1, p, st) : launch_sw<__nv_bfloat16, false, 1>(c, a, 1, p, st);
     if (rc) return rc;
-    c.sdtc_seq += 1;
-    c.sdtc_gen_expect[buf] += (unsigned)heads;
     g_launches.fetch_add(1);
     t_last_path = "splitd_stream";
     return B200ATTN_OK;
@@ -1164,6 +1180,9 @@ void b200attn_release_workspace(void) {
         c.tcw.release();
         c.f32.release();
         c.sw_tables.release();
+        if (c.sw_S) cudaFree(c.sw_S);
+        if (c.sw_cnt) cudaFree(c.sw_cnt);
+        c.sw_S = nullptr; c.sw_cnt = nullptr;
         c.prev_sdtc = false;
     }
     cudaSetDevice(prev);

@@ -10,7 +10,7 @@
 // kernel is bound by its HBM traffic (every input byte is read once) once a CTA has a few blocks; below that by the chain
 // load -> scores -> reduction over the slices -> softmax -> P V -> store that splitd_tc.cuh describes.
 //
-//   warp 0       TMA loads, the scratch buffer's generation, the head's arrival counter
+//   warp 0       TMA loads, the head's arrival counter
 //   warp 1       MMAs
 //   warps 2-7    landed atoms -> (encoding) -> hi | lo operand stage; landed V -> hi and lo (16-bit V: -> its fp32 operand layout)
 //   warps 8-11   partial scores -> scratch, softmax, P, epilogue of each block of 128 output columns
@@ -23,7 +23,9 @@
 // by 1.1e-7 to 1.8e-7, this form by 0.8e-7 to 1.0e-7.  The encoding and the softmax are fp32 as in splitd.cuh.
 // Infinities and NaN: pieces of a non-finite value would turn inf * x into NaN (inf * 0 of a lower piece), so a CTA that meets one
 // in its slice takes plain FFMA loops for what it enters into (its partial scores; its block of output columns).
-// The score scratch is the ring of splitd_tc.cuh (same buffers, counters and generations).
+// The score scratch is one buffer, cleared by its user: a call starts after the one before it in the stream is complete.  (The ring
+// of splitd_tc.cuh, whose generations the host counts, is for calls that overlap; a call captured into a graph is counted there
+// but runs when the graph is launched, never or often, and later calls then waited for a generation that did not come.)
 #pragma once
 
 #include <type_traits>
@@ -59,13 +61,12 @@ struct SwParams {
     int BH;                  // heads of one problem
     int Lq, Lk, D;
     int natoms, nsplit;      // atoms of 32 columns; slices per head
-    int buf, cap_bh;
-    unsigned gen_expect;
     int pe, rd;
     const float2 *tab;       // [64 positions][16 natoms] (cos, sin) of a pair of columns; what leaves a pair alone where it is not encoded
     float scale;
-    float *S;
-    unsigned *counters, *gen, *err, *err_sys;
+    float *S;                // [heads of the launch][64][64]
+    unsigned *counters;      // [heads][2]: warps that have added their scores, warps that have read the sums
+    unsigned *err, *err_sys;
     unsigned spin_limit, wait_extra;
 };
 
@@ -73,7 +74,7 @@ struct SwBars {
     uint64_t full[SW_NR], raw_free[SW_NR];
     uint64_t ready[SW_NST], st_free[SW_NST];
     uint64_t acc_full[2], acc_empty[2];     // a group of atoms has been multiplied / read
-    uint64_t s_full, buf_ok, head_ok, p_ready;
+    uint64_t s_full, head_ok, p_ready;
     uint64_t v_full[SW_NV], v_free[SW_NV];
     uint64_t v_ready[2], vop_free[2];
     uint64_t o_full[2], o_empty[2];
@@ -192,8 +193,8 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
     const int nblk = (nat + 3) >> 2;
     auto atom_col = [&](int c) { return (slice + c * p.nsplit) * ST_ATOM; };
     const uint32_t lim = p.spin_limit;
-    float *S_cur = p.S + ((size_t)p.buf * p.cap_bh + head) * 4096;
-    unsigned *cnt_cur = p.counters + ((size_t)p.buf * p.cap_bh + head) * 2;
+    float *S_cur = p.S + (size_t)head * 4096;
+    unsigned *cnt_cur = p.counters + (size_t)head * 2;
     const CUtensorMap *tmQ = &pr.q[prob], *tmK = &pr.k[prob], *tmV = &pr.v[prob];
 
     auto load_atom = [&](int c, int r) {
@@ -218,7 +219,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
             mbar_init(&bars.o_full[i], 1); mbar_init(&bars.o_empty[i], 4);
         }
         for (int i = 0; i < SW_NV; ++i) { mbar_init(&bars.v_full[i], 1); mbar_init(&bars.v_free[i], 6); }
-        mbar_init(&bars.s_full, 1); mbar_init(&bars.buf_ok, 1); mbar_init(&bars.head_ok, 1); mbar_init(&bars.p_ready, 4);
+        mbar_init(&bars.s_full, 1); mbar_init(&bars.head_ok, 1); mbar_init(&bars.p_ready, 4);
         s_fail = 0u; s_odd_qk = 0u; s_odd_v[0] = s_odd_v[1] = 0u;
         mbar_fence_init();
         grid_dependency_wait();   // (a no-op unless launched as a programmatic dependent)
@@ -238,18 +239,6 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
     if (warp == 0) {
         if (elect_one()) {
             do {
-                // the buffer of the scratch ring is clean once its earlier users have cleared their heads
-                unsigned seen = 0;
-                for (unsigned it = 0; it < lim; ++it) {
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(p.gen + p.buf) : "memory");
-                    if ((int)(seen - p.gen_expect) >= 0) break;
-                    __nanosleep(100);
-                }
-                if ((int)(seen - p.gen_expect) < 0) {
-                    report_kernel_error(p.err, p.err_sys, (unsigned)KERR_HEAD_BARRIER_TIMEOUT | (1u << 20));
-                    *reinterpret_cast<volatile unsigned *>(&s_fail) = 1u;
-                }
-                mbar_arrive(&bars.buf_ok);
                 for (int c = SW_NR, r = 0, par = 0; c < nat; ++c) {
                     SW_FAIL_AT(0, !mbar_wait(&bars.raw_free[r], (uint32_t)par, lim));
                     load_atom(c, r);
@@ -262,7 +251,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                 }
                 // the head's scores are complete when every read-out warp of every slice has arrived
                 const unsigned want = 4u * (unsigned)p.nsplit + p.wait_extra;
-                seen = 0;
+                unsigned seen = 0;
                 for (unsigned it = 0; it < lim; ++it) {
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(cnt_cur) : "memory");
                     if (seen >= want) break;
@@ -454,7 +443,6 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                 if (lane == 0) mbar_arrive(&bars.acc_empty[g & 1]);
             }
             if (failed) break;
-            SW_WARP_WAIT(13, bars.buf_ok, 0);
             if (__any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned *>(&s_fail) != 0u)) { failed = true; break; }
             const int row = 16 * q + lane;
             if (lane < 16 && row < Lq) {
@@ -521,7 +509,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars.p_ready);
-            // this warp has read the head's scores; the last of all slices' warps to say so clears them for the buffer's next user
+            // this warp has read the head's scores; the last of all slices' warps to say so clears them for the next call
             unsigned old = 0;
             if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(cnt_cur + 1) : "memory");
             old = __shfl_sync(0xffffffffu, old, 0);
@@ -530,9 +518,6 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
 #pragma unroll 4
                 for (int i = lane; i < 1024; i += 32) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < 2) cnt_cur[lane] = 0u;
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.gen + p.buf) : "memory");
             }
             // ---- epilogue: the thread of tensor-memory lane 32 q + l holds output column l of atom 4 b + q; the four lanes of a quad
             // transpose 4 rows x 4 columns, so that a store instruction writes whole lines ----

@@ -152,3 +152,36 @@ def test_one_launch_for_several_problems(pkg, cuda, pe, H, Lq, Lk, D, n):
         res = ol.compare(o.cpu().numpy(), ol.attention(Q, K, V, pe=pe))
         assert res["ok"] and res["max_abs"] <= 5e-5, res
     assert ol.compare(o2.cpu().numpy(), ol.attention(probs[1][-1].cpu().numpy(), probs[0][1], probs[0][2], pe=pe))["ok"]
+
+
+@pytest.mark.parametrize("replays", [0, 1, 12])
+def test_captured_calls(pkg, cuda, replays):
+    """Calls captured into a graph, which is then launched never, once or often, do not get in the way of other calls: of this kernel, of a
+    batch and of the kernel whose scratch is a ring (fp32, no encoding)."""
+    Q, K, V = ol.make_qkv(1, 4, 64, 50, 256, 96, "uniform")
+    T = [to_dev(x, cuda) for x in (Q, K, V)]
+    out, s = torch.empty_like(T[0]), torch.cuda.Stream()
+    want = {pe: ol.attention(Q, K, V, pe=pe) for pe in (ol.PE_NONE, ol.PE_ROPE_INTERLEAVED)}
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        pkg.forward(*T, out=out, pe=ol.PE_ROPE_INTERLEAVED)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            for _ in range(10):
+                pkg.forward(*T, out=out, pe=ol.PE_ROPE_INTERLEAVED, flags=pkg.FLAG_ASYNC)
+        assert pkg.last_path() == "splitd_stream"
+        for rep in range(max(1, replays)):
+            if replays:
+                out.zero_()
+                g.replay()
+                s.synchronize()
+                assert ol.compare(out.cpu().numpy(), want[ol.PE_ROPE_INTERLEAVED])["max_abs"] <= 5e-5
+            for pe in (ol.PE_ROPE_INTERLEAVED, ol.PE_NONE):
+                o = [torch.zeros_like(out) for _ in range(5)]
+                pkg.forward_many([pkg.args_for(*T, x, pe=pe, stream=s.cuda_stream, flags=pkg.FLAG_ASYNC) for x in o])
+                # one entry at a time: each of another length of query, so that none share a launch
+                lone = [pkg.forward(T[0][:, :, :n].contiguous(), T[1], T[2], pe=pe, flags=pkg.FLAG_ASYNC) for n in range(55, 64)]
+                s.synchronize()
+                for x, w in [(x, want[pe]) for x in o] + [(x, want[pe][:, :, :x.shape[2]]) for x in lone]:
+                    assert ol.compare(x.cpu().numpy(), w)["max_abs"] <= 5e-5
+    pkg.forward(*T)   # reports what an asynchronous call left behind
