@@ -26,6 +26,10 @@
 // The score scratch is one buffer, cleared by its user: a call starts after the one before it in the stream is complete.  (The ring
 // of splitd_tc.cuh, whose generations the host counts, is for calls that overlap; a call captured into a graph is counted there
 // but runs when the graph is launched, never or often, and later calls then waited for a generation that did not come.)
+// The slices of a head wait for each other's scores, and the launch does not promise that they run together: while another stream's
+// kernel holds some of the SMs, some slices wait for room.  A slice says that it runs (cnt_cur, upper half) when it starts; until all
+// of them have said so the others' patience is some thousands of times the limit of the waits on work that is running, so such a call
+// takes until there is room, as a cooperative launch would.  (Launched as one: 14.3 -> 16.4 us for 4 heads, 64 x 64, head_d 2048, RoPE.)
 #pragma once
 
 #include <type_traits>
@@ -65,7 +69,7 @@ struct SwParams {
     const float2 *tab;       // [64 positions][16 natoms] (cos, sin) of a pair of columns; what leaves a pair alone where it is not encoded
     float scale;
     float *S;                // [heads of the launch][64][64]
-    unsigned *counters;      // [heads][2]: warps that have added their scores, warps that have read the sums
+    unsigned *counters;      // [heads][2]: warps that have added their scores + 65536 x slices that run, warps that have read the sums
     unsigned *err, *err_sys;
     unsigned spin_limit, wait_extra;
 };
@@ -80,6 +84,20 @@ struct SwBars {
     uint64_t o_full[2], o_empty[2];
 };
 
+// What depends on the other slices of the head: longer waits, cut short when the thread that waits for those has given up.
+constexpr uint32_t SW_ROOM = 4096;   // times the poll limit
+__device__ __forceinline__ bool sw_wait_head(uint64_t *bar, uint32_t parity, uint32_t lim, unsigned *fail) {
+    if (mbar_test_wait(bar, parity)) return true;
+    for (unsigned long long it = 0; it < (unsigned long long)lim * SW_ROOM; ++it) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (it > 64) {
+            __nanosleep(32);
+            if ((it & 63) == 0 && *reinterpret_cast<volatile unsigned *>(fail) != 0u) return false;
+        }
+    }
+    return false;
+}
+
 #define SW_FAIL_AT(site, cond)                                                                       \
     if (cond) {                                                                                      \
         report_kernel_error(p.err, p.err_sys, (unsigned)KERR_MBAR_TIMEOUT | (1u << (7 + (site))));   \
@@ -90,7 +108,11 @@ struct SwBars {
 
 // the same for a wait of a whole warp: either all of its lanes go on or none
 #define SW_WARP_WAIT(site, bar, parity)                                                                          \
-    if (!__all_sync(0xffffffffu, mbar_wait(&(bar), (uint32_t)(parity), lim))) {                                  \
+    SW_WARP_ALL(site, mbar_wait(&(bar), (uint32_t)(parity), lim))
+#define SW_WARP_WAIT_HEAD(site, bar, parity)                                                                     \
+    SW_WARP_ALL(site, sw_wait_head(&(bar), (uint32_t)(parity), lim, &s_fail))
+#define SW_WARP_ALL(site, waited)                                                                                \
+    if (!__all_sync(0xffffffffu, waited)) {                                                                      \
         if (lane == 0) report_kernel_error(p.err, p.err_sys, (unsigned)KERR_MBAR_TIMEOUT | (1u << (7 + (site)))); \
         *reinterpret_cast<volatile unsigned *>(&s_fail) = 1u;                                                    \
         failed = true;                                                                                           \
@@ -223,6 +245,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
         s_fail = 0u; s_odd_qk = 0u; s_odd_v[0] = s_odd_v[1] = 0u;
         mbar_fence_init();
         grid_dependency_wait();   // (a no-op unless launched as a programmatic dependent)
+        asm volatile("red.relaxed.gpu.global.add.u32 [%0], 65536;" ::"l"(cnt_cur) : "memory");   // this slice runs
         for (int c = 0; c < nat && c < SW_NR; ++c) load_atom(c, c);
         for (int b = 0; b < nblk && b < 2; ++b) load_v(b, b);
     }
@@ -251,20 +274,22 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                 }
                 // the head's scores are complete when every read-out warp of every slice has arrived
                 const unsigned want = 4u * (unsigned)p.nsplit + p.wait_extra;
-                unsigned seen = 0;
-                for (unsigned it = 0; it < lim; ++it) {
+                unsigned seen = 0, polls = 0;
+                for (unsigned it = 0; polls < lim; ++it) {
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(cnt_cur) : "memory");
-                    if (seen >= want) break;
-                    __nanosleep(20);
+                    if ((seen & 0xffffu) >= want) break;
+                    const bool all = (seen >> 16) == (unsigned)p.nsplit;
+                    __nanosleep(all ? 20 : 500);
+                    if (all || (it & (SW_ROOM / 16 - 1)) == 0) ++polls;   // (some twenty times as long a poll)
                 }
-                if (seen < want) {
+                if ((seen & 0xffffu) < want) {
                     report_kernel_error(p.err, p.err_sys, (unsigned)KERR_HEAD_BARRIER_TIMEOUT);
                     *reinterpret_cast<volatile unsigned *>(&s_fail) = 1u;
                 }
                 mbar_arrive(&bars.head_ok);
-                if (seen < want) break;
+                if ((seen & 0xffffu) < want) break;
                 for (int b = SW_NV, s = 0, par = 0; b < nblk; ++b) {
-                    SW_FAIL_AT(2, !mbar_wait(&bars.v_free[s], (uint32_t)par, lim));
+                    SW_FAIL_AT(2, !sw_wait_head(&bars.v_free[s], (uint32_t)par, lim, &s_fail));
                     load_v(b, s);
                     if (++s == SW_NV) { s = 0; par ^= 1; }
                 }
@@ -306,13 +331,13 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                 if (failed) break;
                 umma_commit(&bars.s_full);
                 // O[:, block]^T = V^T P^T: V the M-major A operand, P1 P2 P3 one K-major B operand; per 16 keys V1 [P1 | P2 | P3], V2 [P1 | P2], V3 P1
-                SW_FAIL_AT(4, !mbar_wait(&bars.p_ready, 0, lim));
+                SW_FAIL_AT(4, !sw_wait_head(&bars.p_ready, 0, lim, &s_fail));
                 const uint32_t iv64 = umma_idesc_bf16(128, 64, 1, 0), iv128 = umma_idesc_bf16(128, 128, 1, 0), iv192 = umma_idesc_bf16(128, 192, 1, 0);
                 const uint64_t dp = umma_desc_k_sw128(smem_u32(p_buf));
                 for (int b = 0; b < nblk; ++b) {
                     const int e = b & 1;
-                    SW_FAIL_AT(5, !mbar_wait(&bars.v_ready[e], (uint32_t)((b >> 1) & 1), lim));
-                    SW_FAIL_AT(6, !mbar_wait(&bars.o_empty[e], (uint32_t)((b >> 1) & 1) ^ 1u, lim));
+                    SW_FAIL_AT(5, !sw_wait_head(&bars.v_ready[e], (uint32_t)((b >> 1) & 1), lim, &s_fail));
+                    SW_FAIL_AT(6, !sw_wait_head(&bars.o_empty[e], (uint32_t)((b >> 1) & 1) ^ 1u, lim, &s_fail));
                     tc_fence_after();
                     const uint32_t va = smem_u32(v_op + (size_t)e * SW_VOP), to = tmem + 256u * (uint32_t)e;
                     for (int k = 0; k < (kpad >> 4); ++k) {
@@ -381,8 +406,8 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                 SW_WARP_WAIT(9, bars.s_full, 0);   // the stages may be overwritten
                 for (int b = 0, s = 0, par = 0; b < nblk; ++b) {
                     const int e = b & 1, na = min(4, nat - 4 * b);
-                    SW_WARP_WAIT(10, bars.v_full[s], par);
-                    SW_WARP_WAIT(11, bars.vop_free[e], ((b >> 1) & 1) ^ 1);
+                    SW_WARP_WAIT_HEAD(10, bars.v_full[s], par);
+                    SW_WARP_WAIT_HEAD(11, bars.vop_free[e], ((b >> 1) & 1) ^ 1);
                     const unsigned char *in = v_slot(s);
                     unsigned char *out = v_op + (size_t)e * SW_VOP;
                     float odd = 0.0f;
@@ -400,7 +425,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                     }
                     if (__any_sync(0xffffffffu, odd != odd)) {
                         // the word still belongs to block b - 2 until its epilogue, which may be in plain loops, has read it
-                        SW_WARP_WAIT(11, bars.o_empty[e], ((b >> 1) & 1) ^ 1);
+                        SW_WARP_WAIT_HEAD(11, bars.o_empty[e], ((b >> 1) & 1) ^ 1);
                         if (lane == 0) *reinterpret_cast<volatile unsigned *>(&s_odd_v[e]) = (unsigned)b + 1u;
                     }
                     fence_proxy_async_smem();
@@ -458,7 +483,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
             __syncwarp();
             if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt_cur) : "memory");
             SW_WARP_WAIT(14, bars.s_full, 0);    // P goes where atoms landed
-            SW_WARP_WAIT(14, bars.head_ok, 0);
+            SW_WARP_WAIT_HEAD(14, bars.head_ok, 0);
             if (__any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned *>(&s_fail) != 0u)) { failed = true; break; }
             // softmax: half a warp per row, four keys per lane; warp w4 owns rows [16 w4, 16 w4 + 16)
             constexpr int RPW = 8;
@@ -523,7 +548,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
             // transpose 4 rows x 4 columns, so that a store instruction writes whole lines ----
             for (int b = 0; b < nblk; ++b) {
                 const int e = b & 1, a = 4 * b + q;
-                SW_WARP_WAIT(15, bars.o_full[e], (b >> 1) & 1);
+                SW_WARP_WAIT_HEAD(15, bars.o_full[e], (b >> 1) & 1);
                 tc_fence_after();
                 const bool plain = *reinterpret_cast<volatile unsigned *>(&s_odd_v[e]) == (unsigned)b + 1u;   // a non-finite value in the block
                 if (a < nat) {
@@ -585,6 +610,8 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
 
 #undef SW_FAIL_AT
 #undef SW_WARP_WAIT
+#undef SW_WARP_WAIT_HEAD
+#undef SW_WARP_ALL
 
 // The angle tables of the encodings in use, kept between calls (64 positions: 4 KB per 16 columns); bounded, the oldest goes first.
 struct SwTables {

@@ -185,3 +185,35 @@ def test_captured_calls(pkg, cuda, replays):
                 for x, w in [(x, want[pe]) for x in o] + [(x, want[pe][:, :, :x.shape[2]]) for x in lone]:
                     assert ol.compare(x.cpu().numpy(), w)["max_abs"] <= 5e-5
     pkg.forward(*T)   # reports what an asynchronous call left behind
+
+
+def test_slices_wait_for_room_beside_another_stream(pkg, cuda):
+    """Another stream's kernel holds most of the SMs for many times as long as a slice waits for slices that run: the call takes until
+    there is room, and succeeds.  A slice that never arrives is still reported, and the next call works."""
+    Q, K, V = ol.make_qkv(1, 4, 64, 64, 1024, 97, "uniform")
+    T = [to_dev(x, cuda) for x in (Q, K, V)]
+    want = ol.attention(Q, K, V, pe=ol.PE_ROPE_INTERLEAVED)
+    pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED)
+    x = torch.rand(100, 1 << 22, device=cuda)   # such a scan runs one block per row
+    x.logcumsumexp(1)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    L = pkg.lib()
+    pkg.set_option(pkg.OPT_SPIN_LIMIT, 1000)    # a millisecond of polls or so
+    try:
+        with torch.cuda.stream(side):
+            x.logcumsumexp(1)
+        got = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED)   # raises where a wait runs out
+        assert pkg.last_path() == "splitd_stream"
+        torch.cuda.synchronize()
+        assert ol.compare(got.cpu().numpy(), want)["max_abs"] <= 5e-5
+        L.b200attn_debug_lost_arrival(1, 20000)
+        with pytest.raises(pkg.B200AttnError) as ei:
+            pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED)
+        assert ei.value.status == 4   # B200ATTN_ERR_KERNEL
+    finally:
+        L.b200attn_debug_lost_arrival(0, 0)
+        pkg.set_option(pkg.OPT_SPIN_LIMIT, 1 << 21)
+        torch.cuda.synchronize()
+    for _ in range(2):
+        assert ol.compare(pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED).cpu().numpy(), want)["max_abs"] <= 5e-5
