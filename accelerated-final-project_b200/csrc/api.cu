@@ -555,7 +555,8 @@ static int ensure_sw_scratch(DeviceCtx &c, cudaStream_t st) {
         c.sw_S = S; c.sw_cnt = cnt;
         c.scratch_dirty = true;   // cleared below, on this call's stream
     }
-    return c.scratch_dirty ? ensure_scratch(c, 0, 0, st) : B200ATTN_OK;
+    // (with the scratch of the CUDA-core kernels: a call under capture whose encoding has no table yet goes to them and cannot allocate)
+    return c.scratch_dirty ? ensure_scratch(c, (size_t)c.sm_count * 4096 * sizeof(float), (size_t)2 * c.sm_count, st) : B200ATTN_OK;
 }
 
 // One launch for `n` (<= SW_MAXP) problems of the same form, n heads' worth of CTAs on the chip at once.  -1: not taken, nothing launched.

@@ -613,29 +613,38 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
 #undef SW_WARP_WAIT_HEAD
 #undef SW_WARP_ALL
 
-// The angle tables of the encodings in use, kept between calls (64 positions: 4 KB per 16 columns); bounded, the oldest goes first.
+// The angle tables of the encodings in use, kept between calls (64 positions: 4 KB per 16 columns).  None is given up for another
+// - a captured call keeps a pointer to its own - so there is an end to them: an encoding beyond it, or one first met while the
+// stream is being captured (its table would be filled when the graph is launched only), has none.
 struct SwTables {
-    struct Entry { float2 *tab = nullptr; int D = 0, rd = 0, sinus = 0; float base = 0.0f; };
-    static constexpr int kEntries = 16;
-    Entry e[kEntries];
-    int next = 0;
+    struct Entry { float2 *tab; int D, rd, sinus; float base; };
+    static constexpr int kEntries = 1024;
+    static constexpr size_t kBytes = (size_t)128 << 20;
+    Entry e[kEntries] = {};
+    int count = 0;
+    size_t bytes = 0;
     const float2 *get(int D, int rd, float base, int sinus, cudaStream_t st, std::atomic<unsigned long long> *launches) {
-        for (const Entry &x : e)
-            if (x.tab && x.D == D && x.rd == rd && x.base == base && x.sinus == sinus) return x.tab;
-        Entry &x = e[next];
-        if (x.tab) { cudaDeviceSynchronize(); cudaFree(x.tab); x.tab = nullptr; }
+        for (int i = count; i-- > 0;)
+            if (e[i].D == D && e[i].rd == rd && e[i].base == base && e[i].sinus == sinus) return e[i].tab;
         const int npairs = 16 * ((D + ST_ATOM - 1) / ST_ATOM);
-        if (cudaMalloc((void **)&x.tab, (size_t)64 * npairs * sizeof(float2)) != cudaSuccess) { (void)cudaGetLastError(); x.tab = nullptr; return nullptr; }
-        sw_table_kernel<<<296, 256, 0, st>>>(x.tab, npairs, D, rd, base, sinus);
+        const size_t n = (size_t)64 * npairs * sizeof(float2);
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (count >= kEntries || bytes + n > kBytes || cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        float2 *tab = nullptr;
+        if (cudaMalloc((void **)&tab, n) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+        sw_table_kernel<<<296, 256, 0, st>>>(tab, npairs, D, rd, base, sinus);
+        if (cudaGetLastError() != cudaSuccess) { cudaFree(tab); return nullptr; }
         launches->fetch_add(1);
-        if (cudaGetLastError() != cudaSuccess) { cudaFree(x.tab); x.tab = nullptr; return nullptr; }
-        x.D = D; x.rd = rd; x.base = base; x.sinus = sinus;
-        next = (next + 1) % kEntries;
-        return x.tab;
+        e[count++] = {tab, D, rd, sinus, base};
+        bytes += n;
+        return tab;
     }
     void release() {
-        for (Entry &x : e) { if (x.tab) cudaFree(x.tab); x = Entry(); }
-        next = 0;
+        while (count > 0) cudaFree(e[--count].tab);
+        bytes = 0;
     }
 };
 

@@ -217,3 +217,43 @@ def test_slices_wait_for_room_beside_another_stream(pkg, cuda):
         torch.cuda.synchronize()
     for _ in range(2):
         assert ol.compare(pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED).cpu().numpy(), want)["max_abs"] <= 5e-5
+
+
+def test_more_encodings_than_are_kept(pkg, cuda):
+    """The tables of angles: a captured call's own stays where it is whatever comes after it, an encoding beyond the last table and one
+    first met under capture run without."""
+    Q, K, V = ol.make_qkv(1, 2, 20, 30, 64, 98, "uniform")
+    T = [to_dev(x, cuda) for x in (Q, K, V)]
+    pe, bases = ol.PE_ROPE_INTERLEAVED, [1000.0 + i for i in range(1100)]
+    wants = {b: ol.attention(Q, K, V, pe=pe, base=b) for b in (bases[0], bases[1], bases[-1], 77.0)}
+    out, out77, s = torch.empty_like(T[0]), torch.empty_like(T[0]), torch.cuda.Stream()
+
+    def check(o, b):
+        assert ol.compare(o.cpu().numpy(), wants[b])["max_abs"] <= 5e-5
+    pkg.lib().b200attn_release_workspace()
+    torch.cuda.synchronize()
+    try:
+        with torch.cuda.stream(s):
+            pkg.forward(*T, out=out, pe=pe, rope_base=bases[0])
+            assert pkg.last_path() == "splitd_stream"
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                pkg.forward(*T, out=out, pe=pe, rope_base=bases[0], flags=pkg.FLAG_ASYNC)
+                assert pkg.last_path() == "splitd_stream"
+                pkg.forward(*T, out=out77, pe=pe, rope_base=77.0, flags=pkg.FLAG_ASYNC)
+                assert pkg.last_path() == "splitd_fused"
+            for b in bases:
+                last = pkg.forward(*T, pe=pe, rope_base=b, flags=pkg.FLAG_ASYNC)
+            assert pkg.last_path() == "splitd_fused"
+            check(last, bases[-1])
+            check(pkg.forward(*T, pe=pe, rope_base=bases[1]), bases[1])
+            assert pkg.last_path() == "splitd_stream"
+            out.zero_()
+            g.replay()
+            s.synchronize()
+            check(out, bases[0])
+            check(out77, 77.0)
+            del g
+    finally:
+        torch.cuda.synchronize()
+        pkg.lib().b200attn_release_workspace()
