@@ -56,13 +56,10 @@ struct F32Params {
     int nq, nk, ndb;           // query tiles, key tiles, blocks of 64 output columns
     int upc;                   // P V kernel: steps of 64 keys per CTA of the cluster
     float c;                   // log2(e) / sqrt(head_d)
-    const __nv_bfloat16 *q, *k, *v;   // planes [pieces][heads][L][Dp]
     float *S;                  // [heads][nq][nk][32 groups of 4 keys][128 rows][4]
     int *rowmax;               // [heads][nq * 128] largest score of a row, as f3_key; the split kernel starts it at the lowest key
     void *O;                   // [heads * Lq][D]
     int vec_out;               // stores of four columns
-    const unsigned *mark;      // == call: a non-finite value has been met
-    unsigned call;
     unsigned *err, *err_sys;
     unsigned spin_limit;
 };
@@ -78,13 +75,10 @@ __device__ __forceinline__ void f3_split2(float x0, float x1, uint32_t &a, uint3
 // fp32 values as integers of the same order (NaN aside), and back
 __device__ __forceinline__ int f3_key(float x) { const int i = __float_as_int(x); return i >= 0 ? i : i ^ 0x7fffffff; }
 __device__ __forceinline__ float f3_unkey(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
-// the value back from its N pieces
-template <int N> __device__ __forceinline__ float f3_join(const __nv_bfloat16 *p, long long plane) {
-    float x = __bfloat162float(p[0]);
-    if (N > 1) x += __bfloat162float(p[plane]);
-    if (N > 2) x += __bfloat162float(p[2 * plane]);
-    return x;
-}
+// The sum of the leading products and the smaller ones.  A sum of leading products that is not finite is the result: of a
+// non-finite operand only the first piece holds it (the others are zero, times which the smaller products are NaN), and of finite
+// operands whose products overflow a lower piece may have the other sign.
+__device__ __forceinline__ float f3_sum(float lead, float small) { return fabsf(lead) < INFINITY ? lead + small : lead; }
 
 // ---- split (and encode) ---------------------------------------------------------------------------
 struct F32SplitTensor {
@@ -93,7 +87,6 @@ struct F32SplitTensor {
     int L;
     int encode;                // the encoding applies to this tensor
     int pieces;
-    int track;                 // its non-finite values must not reach the MMAs (with one piece on either side they may)
 };
 struct F32SplitParams {
     F32SplitTensor t[3];       // blockIdx.z
@@ -103,8 +96,6 @@ struct F32SplitParams {
     const float *cos_cache, *sin_cache;
     int *rowmax;               // nrows entries, set to the key of -inf
     long long nrows;
-    unsigned *mark;
-    unsigned call;
 };
 
 // A thread owns eight columns of one row position and takes a share (gridDim.y) of the heads with them, so that the angles
@@ -120,7 +111,6 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
     const bool sinus = p.pe == PE_SINUSOIDAL, half = pe_pairs_halves(p.pe);
     const bool vec = D % (16 / (int)sizeof(T)) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     const int step = gridDim.y;
-    bool odd = false;   // a non-finite value has been met
     if (blockIdx.z == 0)
         for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < p.nrows; i += (long long)gridDim.x * gridDim.y * blockDim.x)
             p.rowmax[i] = f3_key(-INFINITY);
@@ -192,7 +182,6 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
 #pragma unroll
             for (int e = 0; e < 8; ++e)
                 if ((__float_as_uint(x[e]) & 0x7f800000u) == 0x7f800000u) {   // the value in the first piece (a NaN stays one), zero in the others
-                    odd = odd || t.track;
                     const uint32_t keep = (e & 1) ? 0x0000ffffu : 0xffff0000u;
                     b[e >> 1] &= keep; c[e >> 1] &= keep;
                     if (x[e] != x[e]) a[e >> 1] |= (e & 1) ? 0x00400000u : 0x00000040u;
@@ -211,7 +200,6 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
             if (two) store(h + step, x1);
         }
     }
-    if (odd) *reinterpret_cast<volatile unsigned *>(p.mark) = p.call;
 }
 
 // ---- scores ---------------------------------------------------------------------------------------
@@ -261,12 +249,11 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     grid_dependency_wait();
     bool failed = false;
     const bool skip = *reinterpret_cast<volatile unsigned *>(p.err) != 0;   // an earlier kernel of the call failed
-    const bool plain = *p.mark == p.call;
 
     if (skip) {
         // fall through to the common exit
     } else if (warp == 0) {
-        if (!plain && elect_one()) {
+        if (elect_one()) {
             int s = 0, ph = 0;
             for (int tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x) {
                 const int h = tile / per_head, r = tile - h * per_head, qt = r / p.nk, kt = r - qt * p.nk;
@@ -284,7 +271,7 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (!plain && elect_one()) {
+        if (elect_one()) {
             const uint32_t id128 = umma_idesc_bf16(128, 128, 0, 0), id256 = umma_idesc_bf16(128, 256, 0, 0);
             int s = 0, ph = 0;
             uint32_t g = 0;   // groups so far
@@ -325,36 +312,24 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             float s[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) s[j] = 0.0f;
-            if (plain) {
-                // non-finite values about: the same sums in FFMA, from the planes
-                if (qrow < p.Lq) {
-                    const long long qpl = (long long)p.heads * p.Lq * p.Dp, kpl = (long long)p.heads * p.Lk * p.Dp;
-                    const __nv_bfloat16 *qp = p.q + ((long long)h * p.Lq + qrow) * p.Dp, *kp = p.k + ((long long)h * p.Lk + kt * F3_T + 32 * qr) * p.Dp;
+            for (int c = 0; c < nch; c += 2, ++g) {
+                F3_WARP_WAIT(2, acc_full[g & 1], (g >> 1) & 1);
+                tc_fence_after();
+                const uint32_t ta = tl + 256u * (g & 1);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (j < valid)
-                            for (int d = 0; d < p.D; ++d) s[j] = fmaf(f3_join<NQ>(qp + d, qpl), f3_join<NQ>(kp + (long long)j * p.Dp + d, kpl), s[j]);
+                for (int i = 0; i < 2; ++i) {
+                    uint32_t a[16], b[16];
+                    tmem_ld16(ta + 16 * i, a);
+                    if (NQ > 1) tmem_ld16(ta + 128 + 16 * i, b);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) s[16 * i + j] += NQ > 1 ? f3_sum(__uint_as_float(a[j]), __uint_as_float(b[j])) : __uint_as_float(a[j]);
                 }
-            } else {
-                for (int c = 0; c < nch; c += 2, ++g) {
-                    F3_WARP_WAIT(2, acc_full[g & 1], (g >> 1) & 1);
-                    tc_fence_after();
-                    const uint32_t ta = tl + 256u * (g & 1);
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        uint32_t a[16], b[16];
-                        tmem_ld16(ta + 16 * i, a);
-                        if (NQ > 1) tmem_ld16(ta + 128 + 16 * i, b);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) s[16 * i + j] += NQ > 1 ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[g & 1]);
-                }
-                if (failed) break;
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[g & 1]);
             }
+            if (failed) break;
             if (valid < 32) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
@@ -431,7 +406,6 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
     grid_dependency_wait();
     bool failed = false;
     const bool skip = *reinterpret_cast<volatile unsigned *>(p.err) != 0;
-    const bool plain = *p.mark == p.call;
     // warps 2-17: thread = (query row, set of warps: every other step of keys, half of a step's keys and of the output columns)
     const int wg = warp >= 10 ? 1 : 0, hf = ((warp - 2) >> 2) & 1, q = warp & 3, row = 32 * q + lane;
     const float *S_unit = p.S + ((((long long)h * p.nq + qt) * p.nk) * 32 + 16ll * u0) * F3_T * 4;
@@ -443,7 +417,7 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
     if (skip) {
         // fall through to the common exit
     } else if (warp == 0) {
-        if (!plain && elect_one()) {
+        if (elect_one()) {
             for (int u = 0; u < n; ++u) {
                 const int b = u & 1;
                 F3_FAIL_AT(0, !mbar_wait(&s_empty[b], (uint32_t)((u >> 1) & 1) ^ 1u, lim));
@@ -452,7 +426,7 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
             }
         }
     } else if (warp == 18) {   // (a thread of its own: V waits for MMAs, and the scores of the next step must not wait behind it)
-        if (!plain && elect_one()) {
+        if (elect_one()) {
             for (int u = 0; u < n; ++u) {
                 const int b = u & 1;
                 F3_FAIL_AT(0, !mbar_wait(&v_empty[b], (uint32_t)((u >> 1) & 1) ^ 1u, lim));
@@ -463,7 +437,7 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
             }
         }
     } else if (warp == 1) {
-        if (!plain && elect_one()) {
+        if (elect_one()) {
             const uint32_t id192 = umma_idesc_bf16(128, 192, 0, 1), id128 = umma_idesc_bf16(128, 128, 0, 1), id64 = umma_idesc_bf16(128, 64, 0, 1);
             for (int u = 0; u < n; ++u) {
                 const int b = u & 1;
@@ -493,81 +467,65 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
         const int qrow = qt * F3_T + row;
         float m = 0.0f;   // (rows that do not exist: whatever they hold stays in them and is not stored)
         if (qrow < p.Lq) m = f3_unkey(__ldcg(p.rowmax + (long long)h * p.nq * F3_T + qrow)) * p.c;
-        if (plain) {
-            // non-finite values about: the same sums in FFMA, from the planes of V
-            if (qrow < p.Lq) {
-                const long long vpl = (long long)p.heads * p.Lk * p.Dp;
-                const float4 *sp = reinterpret_cast<const float4 *>(S_unit) + row;
-                for (int u = wg; u < n; u += 2)
-                    for (int j = 0; j < 64 && (u0 + u) * 64 + j < p.Lk; ++j) {
-                        const float e = fast_exp2(fmaf(reinterpret_cast<const float *>(sp + ((long long)u * 16 + (j >> 2)) * F3_T)[j & 3], p.c, -m));
-                        const __nv_bfloat16 *vp = p.v + ((long long)h * p.Lk + (u0 + u) * 64 + j) * p.Dp + db * 64 + 32 * hf;
-                        if (hf == 0) l += e;
+        const uint32_t prow = smem_u32(p_smem + (size_t)wg * F3_PBUF) + (uint32_t)row * 128u, sw = (uint32_t)(row & 7);
+        const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + 256u * (uint32_t)wg + 32u * (uint32_t)hf;
+        const float4 *sp = reinterpret_cast<const float4 *>(s_smem + (size_t)wg * F3_SSTEP) + row;
+        auto fold = [&]() {   // o += the three accumulators of this set
+            tc_fence_after();
 #pragma unroll
-                        for (int d = 0; d < 32; ++d) o[d] = fmaf(e, f3_join<NV>(vp + d, vpl), o[d]);
-                    }
+            for (int g = 0; g < 4; ++g) {
+                uint32_t a[8], b[8], c[8];
+                tmem_ld8(ta + 8 * g, a);
+                tmem_ld8(ta + 64 + 8 * g, b);
+                tmem_ld8(ta + 128 + 8 * g, c);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[8 * g + j] += f3_sum(__uint_as_float(a[j]), __uint_as_float(b[j]) + __uint_as_float(c[j]));
             }
-        } else {
-            const uint32_t prow = smem_u32(p_smem + (size_t)wg * F3_PBUF) + (uint32_t)row * 128u, sw = (uint32_t)(row & 7);
-            const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + 256u * (uint32_t)wg + 32u * (uint32_t)hf;
-            const float4 *sp = reinterpret_cast<const float4 *>(s_smem + (size_t)wg * F3_SSTEP) + row;
-            auto fold = [&]() {   // o += the three accumulators of this set
-                tc_fence_after();
+            tc_fence_before();
+        };
+        int i = 0;   // steps of this set so far
+        for (int u = wg; u < n; u += 2, ++i) {
+            F3_WARP_WAIT(3, s_full[wg], i & 1);
+            float e[32];   // the step's scores of this thread: the stage is free for the next step's at once
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    uint32_t a[8], b[8], c[8];
-                    tmem_ld8(ta + 8 * g, a);
-                    tmem_ld8(ta + 64 + 8 * g, b);
-                    tmem_ld8(ta + 128 + 8 * g, c);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) o[8 * g + j] += __uint_as_float(a[j]) + (__uint_as_float(b[j]) + __uint_as_float(c[j]));
-                }
-                tc_fence_before();
-            };
-            int i = 0;   // steps of this set so far
-            for (int u = wg; u < n; u += 2, ++i) {
-                F3_WARP_WAIT(3, s_full[wg], i & 1);
-                float e[32];   // the step's scores of this thread: the stage is free for the next step's at once
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const float4 v = sp[(8 * hf + c) * F3_T];
-                    e[4 * c] = v.x; e[4 * c + 1] = v.y; e[4 * c + 2] = v.z; e[4 * c + 3] = v.w;
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&s_empty[wg]);
-                float l0 = 0.0f, l1 = 0.0f, l2 = 0.0f, l3 = 0.0f;
-#pragma unroll
-                for (int c = 0; c < 32; c += 4) {
-                    e[c] = fast_exp2(fmaf(e[c], p.c, -m)); e[c + 1] = fast_exp2(fmaf(e[c + 1], p.c, -m));
-                    e[c + 2] = fast_exp2(fmaf(e[c + 2], p.c, -m)); e[c + 3] = fast_exp2(fmaf(e[c + 3], p.c, -m));
-                    l0 += e[c]; l1 += e[c + 1]; l2 += e[c + 2]; l3 += e[c + 3];
-                }
-                l += (l0 + l1) + (l2 + l3);
-                if (i > 0) {
-                    F3_WARP_WAIT(3, pv_done[wg], (i - 1) & 1);   // P may be overwritten, the products are there
-                    fold();
-                }
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {   // eight keys, 16 bytes of a row of each piece of P
-                    uint32_t a[4], b[4], d[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) f3_split2(e[8 * c + 2 * k], e[8 * c + 2 * k + 1], a[k], b[k], d[k]);
-                    const uint32_t at = prow + (((uint32_t)(4 * hf + c) ^ sw) << 4);
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + F3_SLAB), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]) : "memory");
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 2 * F3_SLAB), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]) : "memory");
-                }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&p_full[wg]);
+            for (int c = 0; c < 8; ++c) {
+                const float4 v = sp[(8 * hf + c) * F3_T];
+                e[4 * c] = v.x; e[4 * c + 1] = v.y; e[4 * c + 2] = v.z; e[4 * c + 3] = v.w;
             }
-            if (!failed && i > 0) {
-                do {
-                    F3_WARP_WAIT(4, pv_done[wg], (i - 1) & 1);
-                    fold();
-                } while (false);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_empty[wg]);
+            float l0 = 0.0f, l1 = 0.0f, l2 = 0.0f, l3 = 0.0f;
+#pragma unroll
+            for (int c = 0; c < 32; c += 4) {
+                e[c] = fast_exp2(fmaf(e[c], p.c, -m)); e[c + 1] = fast_exp2(fmaf(e[c + 1], p.c, -m));
+                e[c + 2] = fast_exp2(fmaf(e[c + 2], p.c, -m)); e[c + 3] = fast_exp2(fmaf(e[c + 3], p.c, -m));
+                l0 += e[c]; l1 += e[c + 1]; l2 += e[c + 2]; l3 += e[c + 3];
             }
+            l += (l0 + l1) + (l2 + l3);
+            if (i > 0) {
+                F3_WARP_WAIT(3, pv_done[wg], (i - 1) & 1);   // P may be overwritten, the products are there
+                fold();
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {   // eight keys, 16 bytes of a row of each piece of P
+                uint32_t a[4], b[4], d[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) f3_split2(e[8 * c + 2 * k], e[8 * c + 2 * k + 1], a[k], b[k], d[k]);
+                const uint32_t at = prow + (((uint32_t)(4 * hf + c) ^ sw) << 4);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + F3_SLAB), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]) : "memory");
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 2 * F3_SLAB), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]) : "memory");
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_full[wg]);
+        }
+        if (!failed && i > 0) {
+            do {
+                F3_WARP_WAIT(4, pv_done[wg], (i - 1) & 1);
+                fold();
+            } while (false);
         }
     }
     if (failed) for (int i = 0; i < 2000; ++i) __nanosleep(1000);
@@ -626,13 +584,10 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
 struct F32Scratch {   // per device, grown on demand
     void *buf = nullptr;
     size_t bytes = 0;
-    unsigned *mark = nullptr;
-    unsigned calls = 0;
     bool attr[3] = {};   // fp32, fp16, bf16
     void release() {
         if (buf) cudaFree(buf);
-        if (mark) cudaFree(mark);
-        buf = nullptr; bytes = 0; mark = nullptr; calls = 0;
+        buf = nullptr; bytes = 0;
     }
 };
 
@@ -687,13 +642,8 @@ inline int f32tc_launch(const b200attn_args &a, int rd, float base, F32Scratch &
         if (cudaMalloc(&sc.buf, want) != cudaSuccess) { (void)cudaGetLastError(); sc.buf = nullptr; return -1; }
         sc.bytes = want;
     }
-    if (!sc.mark) {
-        if (cudaMalloc((void **)&sc.mark, 256) != cudaSuccess) { (void)cudaGetLastError(); sc.mark = nullptr; return -1; }
-        if (cudaMemsetAsync(sc.mark, 0, 256, st) != cudaSuccess) { snprintf(t_tc_error, sizeof t_tc_error, "cudaMemsetAsync failed"); return B200ATTN_ERR_CUDA; }
-    }
     p.c = 1.4426950408889634f / sqrtf((float)D);
     p.vec_out = D % 4 == 0 && ((uintptr_t)a.out & (4 * sizeof(T) - 1)) == 0;
-    p.mark = sc.mark;
     p.err = err_dev; p.err_sys = err_sys; p.spin_limit = spin_limit;
     for (long long h0 = 0; h0 < BH; h0 += G) {
         const int n = (int)(BH - h0 < G ? BH - h0 : G);
@@ -704,20 +654,16 @@ inline int f32tc_launch(const b200attn_args &a, int rd, float base, F32Scratch &
         __nv_bfloat16 *vpl = (__nv_bfloat16 *)b; b += up(n * vb);
         p.S = (float *)b; b += up(n * sb);
         p.rowmax = (int *)b;
-        p.q = qpl; p.k = kpl; p.v = vpl;
         p.heads = n;
         p.O = (T *)a.out + (size_t)h0 * Lq * D;
-        if (++sc.calls == 0) sc.calls = 1;
-        p.call = sc.calls;
         F32SplitParams s{};
         s.heads = n; s.D = D; s.Dp = p.Dp; s.pe = a.pe;
         s.rd = rd; s.base = a.pe == B200ATTN_PE_SINUSOIDAL ? 10000.0f : base;
         s.cos_cache = a.cos_cache; s.sin_cache = a.sin_cache;
-        s.mark = sc.mark; s.call = p.call;
         s.rowmax = p.rowmax; s.nrows = (long long)n * nq * F3_T;
-        s.t[0] = {(const T *)a.Q + (size_t)h0 * Lq * D, qpl, Lq, a.pe != B200ATTN_PE_NONE, nqp, nqp > 1};
-        s.t[1] = {(const T *)a.K + (size_t)h0 * Lk * D, kpl, Lk, pe_encodes_k(a.pe), nqp, nqp > 1};
-        s.t[2] = {(const T *)a.V + (size_t)h0 * Lk * D, vpl, Lk, 0, NV, 1};
+        s.t[0] = {(const T *)a.Q + (size_t)h0 * Lq * D, qpl, Lq, a.pe != B200ATTN_PE_NONE, nqp};
+        s.t[1] = {(const T *)a.K + (size_t)h0 * Lk * D, kpl, Lk, pe_encodes_k(a.pe), nqp};
+        s.t[2] = {(const T *)a.V + (size_t)h0 * Lk * D, vpl, Lk, 0, NV};
         CUtensorMap tmQ, tmK, tmV;
         if (!make_tmap_grouped_heads(&tmQ, qpl, (long long)nqp * n, Lq, p.Dp, F3_T, 1) || !make_tmap_grouped_heads(&tmK, kpl, (long long)nqp * n, Lk, p.Dp, F3_T, 1) ||
             !make_tmap_grouped_heads(&tmV, vpl, (long long)NV * n, Lk, p.Dp, 64, 1)) {

@@ -65,6 +65,53 @@ def test_keys_of_minus_infinity_scores_have_no_weight(pkg, cuda):
     torch.testing.assert_close(got, want, rtol=1e-5, atol=MAX_ABS)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_non_finite_value_stays_where_it_belongs(pkg, cuda, dtype):
+    """It decides the rows and columns it enters into; the others do not change by a bit.  (The pieces of its operand are the value and
+    zeros, so it goes through the MMAs like any other.)"""
+    D = 200   # four column blocks, the last one short
+    T = [torch.randn(1, 3, 300, D, generator=torch.Generator().manual_seed(7 + i)).to(dtype).to(cuda) for i in range(3)]
+    clean = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED)
+    assert pkg.last_path() == "tc_f32"
+    bad = [t.clone() for t in T]
+    bad[0][0, 0, 130, 3] = float("nan")     # a query row
+    bad[1][0, 1, 299, 0] = float("nan")     # a key: every row of its head
+    bad[2][0, 2, 5, 70] = float("inf")      # a value: its column
+    bad[2][0, 2, 260, 7] = float("-inf")
+    got = pkg.forward(*bad, pe=ol.PE_ROPE_INTERLEAVED)
+    assert pkg.last_path() == "tc_f32"
+    assert torch.isnan(got[0, 0, 130]).all() and torch.isnan(got[0, 1]).all()
+    assert torch.isposinf(got[0, 2, :, 70]).all() and torch.isneginf(got[0, 2, :, 7]).all()
+    rows = [i for i in range(300) if i != 130]
+    cols = [c for c in range(D) if c not in (7, 70)]
+    assert torch.equal(got[0, 0, rows], clean[0, 0, rows]) and torch.equal(got[0, 2][:, cols], clean[0, 2][:, cols])
+
+
+def test_replays_of_a_captured_call_are_independent(pkg, cuda):
+    """A replay that meets a non-finite value leaves nothing behind for the next ones."""
+    T = [to_dev(x, cuda) for x in ol.make_qkv(1, 2, 140, 130, 64, 86, "uniform")]
+    keep = [t.clone() for t in T]
+    out, s = torch.empty_like(T[0]), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        want = pkg.forward(*T)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            pkg.forward(*T, out=out, flags=pkg.FLAG_ASYNC)
+            pkg.forward(*T, out=out, flags=pkg.FLAG_ASYNC)
+        for value in (None, float("inf"), None, float("nan"), None):
+            for t, k in zip(T, keep):
+                t.copy_(k)
+                if value is not None:
+                    t[0, 0, 3, 3] = value
+            g.replay()
+            s.synchronize()
+            if value is None:
+                assert torch.equal(out, want)
+            else:
+                assert torch.isnan(out[0, 0]).any() and torch.equal(out[0, 1], want[0, 1])
+
+
 def test_scratch_cap_and_misaligned_tensors(pkg, cuda):
     """Heads go in passes where the scratch cap is small; rows and pointers without 16-byte alignment are taken too."""
     Q, K, V = ol.make_qkv(1, 7, 150, 170, 40, 84, "uniform")
