@@ -49,6 +49,7 @@ constexpr int F3_A_THREADS = 576;            // score kernel: warp 0 loads, warp
 constexpr int F3_B_THREADS = 608;            // P V kernel: the same, warp 0 loads the scores and warp 18 loads V
 constexpr int F3_MAX_CLUSTER = 8;
 constexpr int F3_OPITCH = 68;                // floats per row of the partial output in shared memory
+constexpr float F3_VSCALE = 1.0f / 128;      // V goes through the MMAs this much smaller: 64 of its products add up without overflow
 
 struct F32Params {
     int heads;                 // heads of this pass
@@ -56,6 +57,7 @@ struct F32Params {
     int nq, nk, ndb;           // query tiles, key tiles, blocks of 64 output columns
     int upc;                   // P V kernel: steps of 64 keys per CTA of the cluster
     float c;                   // log2(e) / sqrt(head_d)
+    float share, unshare;      // a power of two not above 1 / (steps of 64 keys): unnormalised sums of finite values stay finite; 1 / (share * F3_VSCALE)
     float *S;                  // [heads][nq][nk][32 groups of 4 keys][128 rows][4]
     int *rowmax;               // [heads][nq * 128] largest score of a row, as f3_key; the split kernel starts it at the lowest key
     void *O;                   // [heads * Lq][D]
@@ -87,6 +89,7 @@ struct F32SplitTensor {
     int L;
     int encode;                // the encoding applies to this tensor
     int pieces;
+    float scale;               // 1, for V F3_VSCALE
 };
 struct F32SplitParams {
     F32SplitTensor t[3];       // blockIdx.z
@@ -177,6 +180,8 @@ __global__ void __launch_bounds__(256) f32_split_kernel(const F32SplitParams p) 
                 }
             }
             uint32_t a[4], b[4], c[4];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] *= t.scale;
 #pragma unroll
             for (int e = 0; e < 4; ++e) f3_split2(x[2 * e], x[2 * e + 1], a[e], b[e], c[e]);
 #pragma unroll
@@ -465,8 +470,9 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
         }
     } else {
         const int qrow = qt * F3_T + row;
+        const bool above = p.c > 1.0f;   // head_d 1 and 2: a finite score times c need not be finite, its distance from the maximum comes first
         float m = 0.0f;   // (rows that do not exist: whatever they hold stays in them and is not stored)
-        if (qrow < p.Lq) m = f3_unkey(__ldcg(p.rowmax + (long long)h * p.nq * F3_T + qrow)) * p.c;
+        if (qrow < p.Lq) m = f3_unkey(__ldcg(p.rowmax + (long long)h * p.nq * F3_T + qrow)) * (above ? 1.0f : p.c);
         const uint32_t prow = smem_u32(p_smem + (size_t)wg * F3_PBUF) + (uint32_t)row * 128u, sw = (uint32_t)(row & 7);
         const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + 256u * (uint32_t)wg + 32u * (uint32_t)hf;
         const float4 *sp = reinterpret_cast<const float4 *>(s_smem + (size_t)wg * F3_SSTEP) + row;
@@ -480,7 +486,7 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
                 tmem_ld8(ta + 128 + 8 * g, c);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[8 * g + j] += f3_sum(__uint_as_float(a[j]), __uint_as_float(b[j]) + __uint_as_float(c[j]));
+                for (int j = 0; j < 8; ++j) o[8 * g + j] = fmaf(f3_sum(__uint_as_float(a[j]), __uint_as_float(b[j]) + __uint_as_float(c[j])), p.share, o[8 * g + j]);
             }
             tc_fence_before();
         };
@@ -496,10 +502,16 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_empty[wg]);
             float l0 = 0.0f, l1 = 0.0f, l2 = 0.0f, l3 = 0.0f;
+            if (above) {   // (the whole grid takes the same branch)
+#pragma unroll
+                for (int c = 0; c < 32; ++c) e[c] = (e[c] - m) * p.c;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 32; ++c) e[c] = fmaf(e[c], p.c, -m);
+            }
 #pragma unroll
             for (int c = 0; c < 32; c += 4) {
-                e[c] = fast_exp2(fmaf(e[c], p.c, -m)); e[c + 1] = fast_exp2(fmaf(e[c + 1], p.c, -m));
-                e[c + 2] = fast_exp2(fmaf(e[c + 2], p.c, -m)); e[c + 3] = fast_exp2(fmaf(e[c + 3], p.c, -m));
+                e[c] = fast_exp2(e[c]); e[c + 1] = fast_exp2(e[c + 1]); e[c + 2] = fast_exp2(e[c + 2]); e[c + 3] = fast_exp2(e[c + 3]);
                 l0 += e[c]; l1 += e[c + 1]; l2 += e[c + 2]; l3 += e[c + 3];
             }
             l += (l0 + l1) + (l2 + l3);
@@ -556,7 +568,7 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
                 sum += (ld_cluster_f32(lpeer) + ld_cluster_f32(lpeer + F3_T * 4)) + (ld_cluster_f32(lpeer + 2 * F3_T * 4) + ld_cluster_f32(lpeer + 3 * F3_T * 4));
                 v.x += x.x + y.x; v.y += x.y + y.y; v.z += x.z + y.z; v.w += x.w + y.w;
             }
-            const float inv = 1.0f / sum;
+            const float inv = p.unshare * (1.0f / sum);
             v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
             T *op = reinterpret_cast<T *>(p.O) + ((long long)h * p.Lq + qrow) * p.D + db * 64 + c;
             if (p.vec_out) {
@@ -643,6 +655,10 @@ inline int f32tc_launch(const b200attn_args &a, int rd, float base, F32Scratch &
         sc.bytes = want;
     }
     p.c = 1.4426950408889634f / sqrtf((float)D);
+    int steps_log2 = 0;
+    while ((64ll << steps_log2) < Lk) ++steps_log2;
+    p.share = ldexpf(1.0f, -steps_log2);
+    p.unshare = 1.0f / (p.share * F3_VSCALE);
     p.vec_out = D % 4 == 0 && ((uintptr_t)a.out & (4 * sizeof(T) - 1)) == 0;
     p.err = err_dev; p.err_sys = err_sys; p.spin_limit = spin_limit;
     for (long long h0 = 0; h0 < BH; h0 += G) {
@@ -661,9 +677,9 @@ inline int f32tc_launch(const b200attn_args &a, int rd, float base, F32Scratch &
         s.rd = rd; s.base = a.pe == B200ATTN_PE_SINUSOIDAL ? 10000.0f : base;
         s.cos_cache = a.cos_cache; s.sin_cache = a.sin_cache;
         s.rowmax = p.rowmax; s.nrows = (long long)n * nq * F3_T;
-        s.t[0] = {(const T *)a.Q + (size_t)h0 * Lq * D, qpl, Lq, a.pe != B200ATTN_PE_NONE, nqp};
-        s.t[1] = {(const T *)a.K + (size_t)h0 * Lk * D, kpl, Lk, pe_encodes_k(a.pe), nqp};
-        s.t[2] = {(const T *)a.V + (size_t)h0 * Lk * D, vpl, Lk, 0, NV};
+        s.t[0] = {(const T *)a.Q + (size_t)h0 * Lq * D, qpl, Lq, a.pe != B200ATTN_PE_NONE, nqp, 1.0f};
+        s.t[1] = {(const T *)a.K + (size_t)h0 * Lk * D, kpl, Lk, pe_encodes_k(a.pe), nqp, 1.0f};
+        s.t[2] = {(const T *)a.V + (size_t)h0 * Lk * D, vpl, Lk, 0, NV, F3_VSCALE};
         CUtensorMap tmQ, tmK, tmV;
         if (!make_tmap_grouped_heads(&tmQ, qpl, (long long)nqp * n, Lq, p.Dp, F3_T, 1) || !make_tmap_grouped_heads(&tmK, kpl, (long long)nqp * n, Lk, p.Dp, F3_T, 1) ||
             !make_tmap_grouped_heads(&tmV, vpl, (long long)NV * n, Lk, p.Dp, 64, 1)) {

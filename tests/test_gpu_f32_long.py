@@ -112,6 +112,31 @@ def test_replays_of_a_captured_call_are_independent(pkg, cuda):
                 assert torch.isnan(out[0, 0]).any() and torch.equal(out[0, 1], want[0, 1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_large_values_stay_finite(pkg, cuda, dtype):
+    """A weighted mean of finite values is finite, whatever their size and number."""
+    T = [torch.rand(1, 2, 300, 72, generator=torch.Generator().manual_seed(9 + i)).to(dtype).to(cuda) for i in range(3)]
+    T[2][0, 1, :, 30:] *= 3.3e38
+    got = pkg.forward(*T)
+    assert pkg.last_path() == "tc_f32"
+    want = pkg.forward(*T, flags=pkg.FLAG_FORCE_GENERIC)
+    assert torch.isfinite(want).all()
+    torch.testing.assert_close(got, want, rtol=1e-5 if dtype == torch.float32 else 2.0 ** -7, atol=MAX_ABS)
+
+
+@pytest.mark.parametrize("D", [1, 2])
+def test_large_scores_of_the_narrowest_heads_stay_finite(pkg, cuda, D):
+    """log2(e) / sqrt(head_d) is above 1: the scaled score of a finite one need not be finite."""
+    T = [torch.rand(1, 2, 100, D, generator=torch.Generator().manual_seed(12 + i)) for i in range(3)]
+    T[0] = torch.full_like(T[0], 1e19)
+    T[1] = torch.full_like(T[1], 3e19 / D)
+    T[1][0, 1, 10:] *= 0.5
+    got = pkg.forward(*(t.to(cuda) for t in T)).cpu()
+    assert pkg.last_path() == "tc_f32"
+    want = torch.stack([T[2][0, 0].mean(0), T[2][0, 1, :10].mean(0)])   # equal scores, and a half of the keys without weight
+    torch.testing.assert_close(got[0], want[:, None].expand(2, 100, D), rtol=1e-5, atol=MAX_ABS)
+
+
 def test_scratch_cap_and_misaligned_tensors(pkg, cuda):
     """Heads go in passes where the scratch cap is small; rows and pointers without 16-byte alignment are taken too."""
     Q, K, V = ol.make_qkv(1, 7, 150, 170, 40, 84, "uniform")
