@@ -77,10 +77,41 @@ __device__ __forceinline__ void f3_split2(float x0, float x1, uint32_t &a, uint3
 // fp32 values as integers of the same order (NaN aside), and back
 __device__ __forceinline__ int f3_key(float x) { const int i = __float_as_int(x); return i >= 0 ? i : i ^ 0x7fffffff; }
 __device__ __forceinline__ float f3_unkey(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
-// The sum of the leading products and the smaller ones.  A sum of leading products that is not finite is the result: of a
-// non-finite operand only the first piece holds it (the others are zero, times which the smaller products are NaN), and of finite
-// operands whose products overflow a lower piece may have the other sign.
-__device__ __forceinline__ float f3_sum(float lead, float small) { return fabsf(lead) < INFINITY ? lead + small : lead; }
+// two fp32 additions, multiply-adds
+__device__ __forceinline__ float2 f3_add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 f3_fma2(float2 a, float b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmov.b64 z, {%5, %6};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 f3_pair(const uint32_t *r) { return make_float2(__uint_as_float(r[0]), __uint_as_float(r[1])); }
+// Sums of the leading products and the smaller ones (low: null or the third set).  A sum of leading products that is not finite is the
+// result: of a non-finite operand only the first piece holds it (the others are zero, times which the smaller products are NaN),
+// and of finite operands whose products overflow a lower piece may have the other sign.  One look for all N: looking at each sum cost the
+// P V kernel 6 % (32 heads, 2048 x 2048, head_d 64, the call 311 -> 332 us).
+template <int N> __device__ __forceinline__ void f3_sums(const uint32_t (&lead)[N], const uint32_t (&mid)[N], const uint32_t *low, float2 (&v)[N / 2]) {
+    float2 look = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        const float2 m = f3_pair(mid + 2 * i);
+        v[i] = f3_add2(f3_pair(lead + 2 * i), low != nullptr ? f3_add2(m, f3_pair(low + 2 * i)) : m);
+        look = f3_fma2(v[i], 0.0f, look);
+    }
+    if (!(look.x + look.y == 0.0f)) {
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            const float2 a = f3_pair(lead + 2 * i);
+            if (!(fabsf(a.x) < INFINITY)) v[i].x = a.x;
+            if (!(fabsf(a.y) < INFINITY)) v[i].y = a.y;
+        }
+    }
+}
 
 // ---- split (and encode) ---------------------------------------------------------------------------
 struct F32SplitTensor {
@@ -327,8 +358,10 @@ f32_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                     tmem_ld16(ta + 16 * i, a);
                     if (NQ > 1) tmem_ld16(ta + 128 + 16 * i, b);
                     tmem_ld_wait();
+                    float2 v[8];
+                    if (NQ > 1) f3_sums<16>(a, b, nullptr, v);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) s[16 * i + j] += NQ > 1 ? f3_sum(__uint_as_float(a[j]), __uint_as_float(b[j])) : __uint_as_float(a[j]);
+                    for (int j = 0; j < 16; ++j) s[16 * i + j] += NQ > 1 ? (j & 1 ? v[j >> 1].y : v[j >> 1].x) : __uint_as_float(a[j]);
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -485,8 +518,13 @@ f32_pv_kernel(const __grid_constant__ CUtensorMap tmV, const F32Params p) {
                 tmem_ld8(ta + 64 + 8 * g, b);
                 tmem_ld8(ta + 128 + 8 * g, c);
                 tmem_ld_wait();
+                float2 v[4];
+                f3_sums<8>(a, b, c, v);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[8 * g + j] = fmaf(f3_sum(__uint_as_float(a[j]), __uint_as_float(b[j]) + __uint_as_float(c[j])), p.share, o[8 * g + j]);
+                for (int j = 0; j < 4; ++j) {
+                    const float2 x = f3_fma2(v[j], p.share, make_float2(o[8 * g + 2 * j], o[8 * g + 2 * j + 1]));
+                    o[8 * g + 2 * j] = x.x; o[8 * g + 2 * j + 1] = x.y;
+                }
             }
             tc_fence_before();
         };
