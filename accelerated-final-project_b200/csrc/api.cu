@@ -538,7 +538,7 @@ static int launch_sw(DeviceCtx &c, const b200attn_args *a, int n, const SwParams
         if (ok) { pr.k[i] = *m; ok = (m = c.tmaps.get(a[i].V, BH * p.Lk, p.D, p.Lk, swz, (int)sizeof(T))) != nullptr; }
         if (!ok) return fail(B200ATTN_ERR_CUDA, "cuTensorMapEncodeTiled failed for the streamed slices");
         pr.v[i] = *m;
-        pr.Q[i] = a[i].Q; pr.K[i] = a[i].K; pr.V[i] = a[i].V; pr.O[i] = a[i].out;
+        pr.O[i] = a[i].out;
     }
     CU_TRY(launch_dependent(sw_kernel<T, PE, NP>, dim3((unsigned)p.nsplit, (unsigned)(n * p.BH)), SW_THREADS, SW_SMEM, 1, st, pr, p));
     return B200ATTN_OK;

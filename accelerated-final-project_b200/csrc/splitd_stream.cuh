@@ -21,8 +21,9 @@
 // these are added up in fp32 registers: the tensor core cuts a sum off where it does not fit, always towards zero.  Against 64
 // bits (uniform inputs, head_d 2048 to 8192) a hi / lo tf32 form of this kernel erred by 6e-7 to 8e-7, the CUDA-core kernels
 // by 1.1e-7 to 1.8e-7, this form by 0.8e-7 to 1.0e-7.  The encoding and the softmax are fp32 as in splitd.cuh.
-// Infinities and NaN: pieces of a non-finite value would turn inf * x into NaN (inf * 0 of a lower piece), so a CTA that meets one
-// in its slice takes plain FFMA loops for what it enters into (its partial scores; its block of output columns).
+// Infinities and NaN go through the MMAs like other values: a sum of leading products that is not finite is the result, whatever
+// the smaller products are (a lower piece of such a value is NaN).  The epilogue looks for such sums only in blocks of V that
+// hold such a value.
 // The score scratch is one buffer, cleared by its user: a call starts after the one before it in the stream is complete.  (The ring
 // of splitd_tc.cuh, whose generations the host counts, is for calls that overlap; a call captured into a graph is counted there
 // but runs when the graph is launched, never or often, and later calls then waited for a generation that did not come.)
@@ -57,7 +58,6 @@ static_assert(SW_NR == 4 && SW_VOP == SW_STAGE && 3 * SW_PL <= 2 * ST_CHUNK && S
 
 template <int NP> struct SwProblems {
     CUtensorMap q[NP], k[NP], v[NP];
-    const void *Q[NP], *K[NP], *V[NP];
     void *O[NP];
 };
 
@@ -171,25 +171,16 @@ template <typename T> __device__ __forceinline__ void sw_open8(const unsigned ch
     }
 }
 
-// ---- the loops taken where a value is not finite ----
-// partial score of row i and key j over the columns of a slice (atoms a0, a0 + step, ...)
-template <typename T, bool PE>
-__device__ __noinline__ float sw_plain_score(const T *q, const T *k, int i, int j, int a0, int step, const SwParams &p) {
-    const bool sinus = p.pe == PE_SINUSOIDAL, enc_k = pe_encodes_k(p.pe);
-    float s = 0.0f;
-    for (int a = a0; a < p.natoms; a += step)
-        for (int c = a * ST_ATOM; c < min(p.D, (a + 1) * ST_ATOM); c += 2) {
-            float q0 = to_f32(q[c]), q1 = to_f32(q[c + 1]), k0 = to_f32(k[c]), k1 = to_f32(k[c + 1]);
-            if (PE && (sinus || c + 1 < p.rd)) {
-                const float2 tq = p.tab[(size_t)i * 16 * p.natoms + (c >> 1)], tk = p.tab[(size_t)j * 16 * p.natoms + (c >> 1)];
-                sw_encode(q0, q1, sinus, tq.x, tq.y);
-                if (enc_k) sw_encode(k0, k1, sinus, tk.x, tk.y);
-            }
-            s = fmaf(q0, k0, s);
-            s = fmaf(q1, k1, s);
-        }
-    return s;
+// The first pieces of eight fp32 values as they landed, some of them not finite: one of a NaN stays a NaN when its low bits are cut off.
+__device__ __noinline__ void sw_keep_nan(const unsigned char *slab, int row, int pc, unsigned char *first) {
+    for (int i = 0; i < 8; ++i)
+        if ((*reinterpret_cast<const uint32_t *>(slab + st_swz(row, 8 * pc + i)) & 0x7fffffffu) > 0x7f800000u) *reinterpret_cast<uint16_t *>(first + 2 * i) |= 0x0040;
 }
+
+// Reports that the head's other slices did not arrive.  (A call that takes the address of the parameters: with one the compiler keeps a copy
+// of them at hand, without it reads them from the constant bank, beside up to 6 KB of tensor maps: 16 problems of 4 heads, 64 x 64,
+// head_d 2048 take 43.1 us with it and 47.6 us without.)
+__device__ __noinline__ void sw_report(const SwParams &p, unsigned bits) { report_kernel_error(p.err, p.err_sys, bits); }
 
 template <typename T, bool PE, int NP>
 __global__ void __launch_bounds__(SW_THREADS, 1)
@@ -202,7 +193,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
     extern __shared__ __align__(256) unsigned char sw_smem_raw[];
     __shared__ SwBars bars;
     __shared__ uint32_t tmem_slot;
-    __shared__ unsigned s_fail, s_odd_qk, s_odd_v[2];   // a non-finite value in Q or K; in block n of V: n + 1
+    __shared__ unsigned s_fail, s_odd_v[2];   // a non-finite value in block n of V: n + 1
     unsigned char *smem = sw_smem_raw + ((1024u - (smem_u32(sw_smem_raw) & 1023u)) & 1023u);
     unsigned char *stages = smem + 2 * SW_VBLK, *raw = stages + 2 * SW_STAGE;
     unsigned char *v_op = stages, *p_buf = raw;
@@ -242,7 +233,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
         }
         for (int i = 0; i < SW_NV; ++i) { mbar_init(&bars.v_full[i], 1); mbar_init(&bars.v_free[i], 6); }
         mbar_init(&bars.s_full, 1); mbar_init(&bars.head_ok, 1); mbar_init(&bars.p_ready, 4);
-        s_fail = 0u; s_odd_qk = 0u; s_odd_v[0] = s_odd_v[1] = 0u;
+        s_fail = 0u; s_odd_v[0] = s_odd_v[1] = 0u;
         mbar_fence_init();
         grid_dependency_wait();   // (a no-op unless launched as a programmatic dependent)
         asm volatile("red.relaxed.gpu.global.add.u32 [%0], 65536;" ::"l"(cnt_cur) : "memory");   // this slice runs
@@ -283,7 +274,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                     if (all || (it & (SW_ROOM / 16 - 1)) == 0) ++polls;   // (some twenty times as long a poll)
                 }
                 if ((seen & 0xffffu) < want) {
-                    report_kernel_error(p.err, p.err_sys, (unsigned)KERR_HEAD_BARRIER_TIMEOUT);
+                    sw_report(p, (unsigned)KERR_HEAD_BARRIER_TIMEOUT);
                     *reinterpret_cast<volatile unsigned *>(&s_fail) = 1u;
                 }
                 mbar_arrive(&bars.head_ok);
@@ -375,6 +366,8 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
             const unsigned char *src = raw + (size_t)r * ST_CHUNK;
             unsigned char *dst = stages + (size_t)(j >> 1) * SW_STAGE;
             float odd = 0.0f;
+            auto first = [&](int op, int row, int pc) { return dst + op * 3 * SW_PL + row * 128 + (((4 * (j & 1) + pc) ^ (row & 7)) << 4); };
+            const bool part = !sinus && atom_col(c) + ST_ATOM > p.rd;   // pairs from rotary_dim on are left alone, infinities too
 #pragma unroll
             for (int n = 0; n < 3; ++n) {
                 const int idx = t + n * SW_SPLIT, op = idx >> 8, row = (idx >> 2) & 63, pc = idx & 3;
@@ -382,20 +375,25 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                     float x[8];
                     sw_open8<T>(src + op * ST_SLAB, row, pc, x);
                     if (PE && (!op || enc_k)) {
+                        const int left = part ? p.rd - (atom_col(c) + 8 * pc) : 8;
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
-                            sw_encode(x[4 * e], x[4 * e + 1], sinus, ang[n][e].x, ang[n][e].y);
-                            sw_encode(x[4 * e + 2], x[4 * e + 3], sinus, ang[n][e].z, ang[n][e].w);
+                            if (4 * e < left) sw_encode(x[4 * e], x[4 * e + 1], sinus, ang[n][e].x, ang[n][e].y);
+                            if (4 * e + 2 < left) sw_encode(x[4 * e + 2], x[4 * e + 3], sinus, ang[n][e].z, ang[n][e].w);
                         }
                     }
                     uint4 w[NQP];
                     odd += sw_pieces<NQP>(x, w);
-                    unsigned char *d = dst + op * 3 * SW_PL + row * 128 + (((4 * (j & 1) + pc) ^ (row & 7)) << 4);
+                    unsigned char *d = first(op, row, pc);
 #pragma unroll
                     for (int i = 0; i < NQP; ++i) *reinterpret_cast<uint4 *>(d + i * SW_PL) = w[i];
                 }
             }
-            if (NQP > 1 && odd != odd) *reinterpret_cast<volatile unsigned *>(&s_odd_qk) = 1u;
+            if (W && odd != odd)
+                for (int idx = t; idx < 512; idx += SW_SPLIT) {
+                    const int op = idx >> 8, row = (idx >> 2) & 63, pc = idx & 3;
+                    if (row < (op ? Lk : Lq)) sw_keep_nan(src + op * ST_SLAB, row, pc, first(op, row, pc));
+                }
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) { mbar_arrive(&bars.ready[j]); mbar_arrive(&bars.raw_free[r]); }
@@ -411,6 +409,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                     const unsigned char *in = v_slot(s);
                     unsigned char *out = v_op + (size_t)e * SW_VOP;
                     float odd = 0.0f;
+                    auto first = [&](int a, int row, int pc) { return out + (a >> 1) * SW_PL + row * 128 + (((4 * (a & 1) + pc) ^ (row & 7)) << 4); };
                     for (int idx = t; idx < (na << 8); idx += SW_SPLIT) {
                         const int a = idx >> 8, row = (idx >> 2) & 63, pc = idx & 3;
                         if (row < kpad) {
@@ -418,13 +417,18 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                             if (row < Lk) sw_open8<T>(in + a * ASLAB, row, pc, x);
                             uint4 w[NVP];
                             odd += sw_pieces<NVP>(x, w);
-                            unsigned char *d = out + (a >> 1) * SW_PL + row * 128 + (((4 * (a & 1) + pc) ^ (row & 7)) << 4);
+                            unsigned char *d = first(a, row, pc);
 #pragma unroll
                             for (int i = 0; i < NVP; ++i) *reinterpret_cast<uint4 *>(d + i * 2 * SW_PL) = w[i];
                         }
                     }
                     if (__any_sync(0xffffffffu, odd != odd)) {
-                        // the word still belongs to block b - 2 until its epilogue, which may be in plain loops, has read it
+                        if (W)
+                            for (int idx = t; idx < (na << 8); idx += SW_SPLIT) {
+                                const int a = idx >> 8, row = (idx >> 2) & 63, pc = idx & 3;
+                                if (row < Lk) sw_keep_nan(in + a * ASLAB, row, pc, first(a, row, pc));
+                            }
+                        // the word still belongs to block b - 2 until its epilogue has read it
                         SW_WARP_WAIT_HEAD(11, bars.o_empty[e], ((b >> 1) & 1) ^ 1);
                         if (lane == 0) *reinterpret_cast<volatile unsigned *>(&s_odd_v[e]) = (unsigned)b + 1u;
                     }
@@ -439,7 +443,6 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
         // ---- warps 8-11, one quadrant of tensor-memory lanes each ----
         const int q = warp & 3, w4 = warp - 8;
         const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16);
-        const T *Qh = reinterpret_cast<const T *>(pr.Q[prob]) + (long long)bh * Lq * p.D, *Kh = reinterpret_cast<const T *>(pr.K[prob]) + (long long)bh * Lk * p.D;
         do {
             // partial scores (M = 64: row r is in lane 32 (r / 16) + r % 16): summed over the groups of atoms, then added to the head's in the scratch
             float acc[64];
@@ -472,13 +475,8 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
             const int row = 16 * q + lane;
             if (lane < 16 && row < Lq) {
                 float *srow = S_cur + (size_t)row * 64;
-                if (NQP > 1 && *reinterpret_cast<volatile unsigned *>(&s_odd_qk) != 0u) {   // a non-finite value in this slice
-                    for (int j = 0; j < Lk; ++j)
-                        atomicAdd(srow + j, sw_plain_score<T, PE>(Qh + (long long)row * p.D, Kh + (long long)j * p.D, row, j, slice, p.nsplit, p));
-                } else {
 #pragma unroll
-                    for (int j = 0; j < 64; j += 4) red_add_v4(srow + j, acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-                }
+                for (int j = 0; j < 64; j += 4) red_add_v4(srow + j, acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
             }
             __syncwarp();
             if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt_cur) : "memory");
@@ -550,7 +548,7 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                 const int e = b & 1, a = 4 * b + q;
                 SW_WARP_WAIT_HEAD(15, bars.o_full[e], (b >> 1) & 1);
                 tc_fence_after();
-                const bool plain = *reinterpret_cast<volatile unsigned *>(&s_odd_v[e]) == (unsigned)b + 1u;   // a non-finite value in the block
+                const bool odd = __any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned *>(&s_odd_v[e]) == (unsigned)b + 1u);   // a non-finite value in the block
                 if (a < nat) {
                     const uint32_t ta = tq + 256u * (uint32_t)e;
                     const int col0 = atom_col(a) + (lane & ~3);   // head_d is a multiple of 4: the four columns are inside or outside together
@@ -564,19 +562,12 @@ sw_kernel(const __grid_constant__ SwProblems<NP> pr, const SwParams p) {
                         float v[16];
 #pragma unroll
                         for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(x0[j]) + (__uint_as_float(x1[j]) + __uint_as_float(x2[j]));
-                        if (plain) {
-                            const int col = min(atom_col(a) + lane, p.D - 1);
-                            const T *vp = reinterpret_cast<const T *>(pr.V[prob]) + (long long)bh * Lk * p.D + col;
+                        if (odd) {   // (the leading products once more: held on to, they cost every block)
+                            tmem_ld16(ta + n0, x0);
+                            tmem_ld_wait();
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                v[j] = 0.0f;
-                                if (n0 + j < Lq)
-                                    for (int k = 0; k < Lk; ++k) {
-                                        const unsigned char *pp = p_buf + (n0 + j) * 128 + (((k >> 3) ^ ((n0 + j) & 7)) << 4) + (k & 7) * 2;
-                                        auto piece = [&](int n) { return __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(pp + n * SW_PL)); };
-                                        v[j] = fmaf((piece(0) + piece(1)) + piece(2), to_f32(vp[(long long)k * p.D]), v[j]);
-                                    }
-                            }
+                            for (int j = 0; j < 16; ++j)
+                                if (!(fabsf(__uint_as_float(x0[j])) < INFINITY)) v[j] = __uint_as_float(x0[j]);
                         }
 #pragma unroll
                         for (int t4 = 0; t4 < 4; ++t4) {

@@ -96,6 +96,19 @@ def test_non_finite_values_as_on_the_cuda_cores(pkg, cuda, dtype, which, value):
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_infinities_beyond_rotary_dim(pkg, cuda, dtype):
+    """A column that is not rotated does not meet its neighbour's infinity (times a sine of 0): a key with a score of -inf has no weight."""
+    T = [to_dev(x, cuda).to(dtype) for x in ol.make_qkv(1, 3, 50, 50, 304, 99, "uniform")]
+    T[0][..., 100].abs_().clamp_(min=0.1)
+    T[1][0, 1, 7, 100] = float("-inf")
+    got = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED, rotary_dim=100)
+    assert pkg.last_path() == "splitd_stream"
+    want = pkg.forward(*T, pe=ol.PE_ROPE_INTERLEAVED, rotary_dim=100, flags=pkg.FLAG_FORCE_GENERIC)
+    assert torch.isfinite(want).all()
+    torch.testing.assert_close(got, want, rtol=1e-5 if dtype == torch.float32 else 2.0 ** -7, atol=MAX_ABS)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("H,D,L", [(148, 512, 64), (148, 640, 33), (20, 4096, 64)])
 def test_non_finite_values_in_many_blocks(pkg, cuda, dtype, H, D, L):
