@@ -379,6 +379,16 @@ static int ensure_ring(DeviceCtx &c, cudaStream_t st) {
     return c.scratch_dirty ? ensure_scratch(c, 0, 0, st) : B200ATTN_OK;
 }
 
+// Atoms of a slice of the kernel of splitd_tc.cuh; -1 where it does not take the call.
+static int sdtc_atoms(const DeviceCtx &c, const b200attn_args &a) {
+    const long long BH = (long long)a.batch_sz * a.num_heads;
+    if (a.dtype != B200ATTN_F32 || a.pe != B200ATTN_PE_NONE || a.len_q > 64 || a.len_k > 64 || a.head_d % 4 != 0) return -1;
+    if ((((uintptr_t)a.Q | (uintptr_t)a.K | (uintptr_t)a.V) & 15) != 0 || ((uintptr_t)a.out & 31) != 0) return -1;   // 32-byte output stores
+    if (BH > c.sm_count || BH > 65535) return -1;
+    const int natoms = (a.head_d + ST_ATOM - 1) / ST_ATOM, slots = (int)(c.sm_count / BH), apc = (natoms + slots - 1) / slots;
+    return apc <= ST_MAX_ATOMS ? apc : -1;
+}
+
 #ifdef B200ATTN_DEVTOOLS
 static float *g_sdtc_dbg = nullptr;
 static unsigned long long *g_sdtc_stamps = nullptr;
@@ -393,16 +403,12 @@ static long long g_sdtc_stamp_calls = 0;   // with B200ATTN_SDTC_STAMP_STRIDE se
 static int run_sdtc(DeviceCtx &c, const b200attn_args &a, cudaStream_t st, bool independent_of_prev, bool batched) {
     const long long BH = (long long)a.batch_sz * a.num_heads;
     const int Lq = a.len_q, Lk = a.len_k, D = a.head_d;
-    if (a.dtype != B200ATTN_F32 || a.pe != B200ATTN_PE_NONE || Lq > 64 || Lk > 64 || D % 4 != 0) return -1;
-    if ((((uintptr_t)a.Q | (uintptr_t)a.K | (uintptr_t)a.V) & 15) != 0 || ((uintptr_t)a.out & 31) != 0) return -1;   // 32-byte output stores
-    if (BH > c.sm_count || BH > 65535) return -1;
+    int apc = sdtc_atoms(c, a);
+    if (apc < 0) return -1;
     const int natoms = (D + ST_ATOM - 1) / ST_ATOM;
-    const int slots = (int)(c.sm_count / BH);
-    int apc = (natoms + slots - 1) / slots;
 #ifdef B200ATTN_DEVTOOLS
     if (const char *e = getenv("B200ATTN_SDTC_APC")) apc = atoi(e);
 #endif
-    if (apc > ST_MAX_ATOMS) return -1;
     const int nsplit = (natoms + apc - 1) / apc;
     // Overlap with the previous call: this call's inputs must not be that call's output.  (Two CTAs
     // share an SM up to half of its shared memory, i.e. with slices of up to 128 columns; the whole of this
@@ -776,31 +782,61 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
 
 // How many of the `n` entries from `a` on go out in one launch of the streamed split-head_d kernel: asynchronous fp32 entries
 // of one form on one stream, none of which touches another's output (entries are independent by contract, but an entry
-// that reads an earlier one's output has always been ordered after it), with at most a CTA per SM in all.  1: not a group.
-static int batch_group(const b200attn_args *a, int n) {
+// that reads an earlier one's output has always been ordered after it), with at most a CTA per SM in all.  1: not a group, and
+// neither are the entries up to a[*run).
+//
+// The alternative of entries that splitd_tc.cuh takes is its chain of overlapping calls.  Groups of four and more beat it 1.2 to 3 times,
+// but not a group that leaves a third of the SMs out while the others have long slices, nor a call or two left over: those have nothing to
+// overlap with.  So such a run goes out in equal groups or not at all.  Measured, chain / groups: fp32, 64 x 64, 3 entries of 60 heads,
+// head_d 256 (2 + 1) 24 / 37 us; 5 of 32, head_d 512 (4 + 1) 40 / 46 us; 5 of 16 heads, head_d 2048 (a slice a head, 80 CTAs) 69 / 76 us;
+// 2 of 40 heads, head_d 512 22 / 24 us; for: 2 of 16 heads, head_d 512 15.5 / 14.0 us; 4 of 32, head_d 512 36 / 26 us; 16 of 4, head_d 2048
+// 87 / 43 us.  Other entries (wide slices, encodings) have a launch each otherwise and take the largest group that fills the chip.
+static int batch_group(const b200attn_args *a, int n, int *run) {
     int rd, rd1; float base, base1;
     DeviceCtx *c;
+    *run = 1;
     if (n < 2 || a->struct_size != sizeof *a || a->dtype != B200ATTN_F32 || !(a->flags & B200ATTN_FLAG_ASYNC) ||
         (a->flags & (B200ATTN_FLAG_FORCE_GENERIC | B200ATTN_FLAG_FORCE_TWO_PASS)))
         return 1;
     if (validate(a, &rd, &base) || get_ctx(&c) || !sw_supported(*c, *a)) return 1;
     const long long BH = (long long)a->batch_sz * a->num_heads;
-    long long most = c->sm_count / BH;
-    if (most > SW_MAXP) most = SW_MAXP;
-    const size_t qb = (size_t)BH * a->len_q * a->head_d * 4, kb = (size_t)BH * a->len_k * a->head_d * 4;
-    auto meet = [](const void *x, size_t nx, const void *y, size_t ny) { return (uintptr_t)x < (uintptr_t)y + ny && (uintptr_t)y < (uintptr_t)x + nx; };
-    int g = 1;
-    for (; g < n && g < most; ++g) {
-        const b200attn_args &b = a[g];
+    const bool chain = sdtc_atoms(*c, *a) > 0;
+    int N = 1;   // entries of this form
+    for (; N < n; ++N) {
+        const b200attn_args &b = a[N];
         if (b.struct_size != sizeof b || b.dtype != a->dtype || b.flags != a->flags || (b.flags & B200ATTN_FLAG_NO_OVERLAP) || b.stream != a->stream || b.pe != a->pe ||
             (long long)b.batch_sz * b.num_heads != BH || b.len_q != a->len_q || b.len_k != a->len_k || b.head_d != a->head_d || b.cos_cache != a->cos_cache)
             break;
-        if (validate(&b, &rd1, &base1) || rd1 != rd || base1 != base || !sw_supported(*c, b)) break;
-        bool apart = true;
-        for (int i = 0; i < g && apart; ++i)
-            apart = !meet(a[i].out, qb, b.out, qb) && !meet(a[i].out, qb, b.Q, qb) && !meet(a[i].out, qb, b.K, kb) && !meet(a[i].out, qb, b.V, kb) &&
-                    !meet(b.out, qb, a[i].Q, qb) && !meet(b.out, qb, a[i].K, kb) && !meet(b.out, qb, a[i].V, kb);
-        if (!apart) break;
+        if (validate(&b, &rd1, &base1) || rd1 != rd || base1 != base || !sw_supported(*c, b) || (sdtc_atoms(*c, b) > 0) != chain) break;
+    }
+    *run = N;
+    int most = (int)(c->sm_count / BH);
+    if (most > SW_MAXP) most = SW_MAXP;
+    if (most < 2 || N < 2) return 1;
+    const int natoms = (a->head_d + ST_ATOM - 1) / ST_ATOM;
+    auto pays = [&](int g) {
+        const int slots = (int)(c->sm_count / (g * BH)), per = (natoms + slots - 1) / slots;   // atoms of a slice
+        const double fill = (double)g * BH * natoms / ((double)c->sm_count * per);
+        return fill >= 0.8 || per <= 8 || (g >= 4 && (fill >= 0.65 || per <= 32));
+    };
+    int g;
+    if (chain) {
+        const int k = (N + most - 1) / most;
+        g = (N + k - 1) / k;
+        if ((k > 1 && N / k < 3) || !pays(g) || !pays(N / k)) return 1;
+    } else {
+        for (g = N < most ? N : most; g > 1 && !pays(g); --g) {}
+        if (g == 1) return 1;
+    }
+    const size_t qb = (size_t)BH * a->len_q * a->head_d * 4, kb = (size_t)BH * a->len_k * a->head_d * 4;
+    auto meet = [](const void *x, size_t nx, const void *y, size_t ny) { return (uintptr_t)x < (uintptr_t)y + ny && (uintptr_t)y < (uintptr_t)x + nx; };
+    *run = 1;
+    for (int m = 1; m < g; ++m) {
+        const b200attn_args &b = a[m];
+        for (int i = 0; i < m; ++i)
+            if (meet(a[i].out, qb, b.out, qb) || meet(a[i].out, qb, b.Q, qb) || meet(a[i].out, qb, b.K, kb) || meet(a[i].out, qb, b.V, kb) ||
+                meet(b.out, qb, a[i].Q, qb) || meet(b.out, qb, a[i].K, kb) || meet(b.out, qb, a[i].V, kb))
+                return m;
     }
     return g;
 }
@@ -920,8 +956,10 @@ int b200attn_debug_tc_prof(unsigned long long *out32, int reset) {
 
 int b200attn_forward_many(const b200attn_args *args, int n) {
     if (args == nullptr || n < 0) return fail(B200ATTN_ERR_INVALID_ARG, "b200attn_forward_many: NULL args or negative n");
+    int alone = 0;   // entries before this one go out by themselves
     for (int i = 0; i < n; ++i) {
-        const int g = batch_group(args + i, n - i);
+        int run = 1, g = 1;
+        if (i >= alone && (g = batch_group(args + i, n - i, &run)) == 1) alone = i + run;
         if (g > 1) {
             int rc = forward_device(&args[i], false, false, g);
             if (rc == B200ATTN_OK) { i += g - 1; continue; }

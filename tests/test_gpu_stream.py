@@ -144,9 +144,17 @@ def test_keys_of_minus_infinity_scores_have_no_weight(pkg, cuda, dtype, pe, H, D
 
 
 @pytest.mark.parametrize("pe", [ol.PE_NONE, ol.PE_SINUSOIDAL])
-@pytest.mark.parametrize("H,Lq,Lk,D,n", [(4, 64, 64, 512, 5), (1, 16, 64, 64, 17), (30, 33, 20, 1000, 6), (148, 8, 8, 64, 2)])
-def test_one_launch_for_several_problems(pkg, cuda, pe, H, Lq, Lk, D, n):
+@pytest.mark.parametrize("H,Lq,Lk,D,n,launches", [
+    (4, 64, 64, 512, 5, (2, 2)),       # five, and the one that reads an output of theirs
+    (1, 16, 64, 64, 17, (2, 2)),       # 9 + 9; encoded 16 + 2
+    (1, 33, 64, 256, 16, (2, 2)),      # 9 + 8; 16 + 1
+    (30, 33, 20, 1000, 6, (7, 3)),     # 4 + 3 would leave SMs out, the overlapping calls are faster; 4 + 2 + 1
+    (60, 16, 16, 256, 2, (3, 2)),      # 2 + 1 the same
+    (148, 8, 8, 64, 2, (3, 3))])       # a head per SM
+def test_one_launch_for_several_problems(pkg, cuda, pe, H, Lq, Lk, D, n, launches):
     """Equal entries of a batch share launches; an entry that reads an earlier one's output still sees it."""
+    if torch.cuda.get_device_properties(cuda).multi_processor_count != 148:
+        pytest.skip("the groups are those of 148 SMs")
     probs, args = [], []
     for i in range(n):
         Q, K, V = ol.make_qkv(1, H, Lq, Lk, D, 100 + i, "uniform")
@@ -155,12 +163,16 @@ def test_one_launch_for_several_problems(pkg, cuda, pe, H, Lq, Lk, D, n):
         args.append(pkg.args_for(q, k, v, probs[-1][-1], pe=pe, flags=pkg.FLAG_ASYNC))
     o2 = torch.full_like(probs[0][3], float("nan"))
     args.append(pkg.args_for(probs[1][-1], probs[0][4], probs[0][5], o2, pe=pe, flags=pkg.FLAG_ASYNC))
+    pkg.forward(*probs[0][3:6], pe=pe)   # (builds the table of angles)
     n0 = pkg.launch_count()
     for _ in range(2):
         pkg.forward_many(args)
     torch.cuda.synchronize()
-    if n * H <= 16:
-        assert pkg.launch_count() - n0 < 2 * len(args)
+    assert pkg.launch_count() - n0 == 2 * launches[pe != ol.PE_NONE]
+    if H < 30:
+        pkg.forward_many(args[:2])
+        assert pkg.last_path() == "splitd_stream"
+    torch.cuda.synchronize()
     for Q, K, V, _, _, _, o in probs:
         res = ol.compare(o.cpu().numpy(), ol.attention(Q, K, V, pe=pe))
         assert res["ok"] and res["max_abs"] <= 5e-5, res
