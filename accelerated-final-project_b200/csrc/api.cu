@@ -531,6 +531,22 @@ static bool sw_supported(const DeviceCtx &c, const b200attn_args &a) {
     return BH <= c.sm_count;
 }
 
+// Where the CUDA-core kernel (one cooperative launch, a slice per SM) is faster than the streamed one: work that is over before a pipeline
+// pays.  us there / here - up to 8 rows in slices of 7 and 8 atoms: 16 heads, 8 x 8, head_d 2048, fp32 RoPE 13.4 / 14.1, 148 heads, 1 x 1,
+// head_d 256, fp32 RoPE 12.4 / 13.9; 16 bit without an encoding, where a head is one slice: 148 heads, 16 x 16, head_d 64 8.3 / 9.2, or over 100 of them:
+// 1 head, 16 x 16, head_d 8192 10.4 / 11.3.  Beside the lines: 16 heads, 12 x 12, head_d 2048, fp32 RoPE 15.3 / 14.7; 75 heads, 20 x 20, head_d 128, bf16
+// 10.4 / 10.0; 148 heads, 40 x 40, head_d 32 10.3 / 9.7; 1 head, 40 x 40, head_d 8192 14.5 / 12.3.  From 40 rows on this one is 1.1 to 2.1 times faster, and
+// several times where a slice is too wide for that kernel.
+static bool sw_slower(const DeviceCtx &c, const b200attn_args &a) {
+    const int natoms = (a.head_d + ST_ATOM - 1) / ST_ATOM, slots = (int)(c.sm_count / ((long long)a.batch_sz * a.num_heads)), per = (natoms + slots - 1) / slots;
+    const int rows = a.len_q > a.len_k ? a.len_q : a.len_k;
+    if (per > 8) return false;   // (a slice of more columns than that kernel takes)
+    if (rows <= 8 && per >= 7) return true;
+    if (a.dtype == B200ATTN_F32 || a.pe != B200ATTN_PE_NONE) return false;
+    if (slots == 1) return rows <= (natoms <= 2 ? 32 : 16);
+    return (natoms + per - 1) / per > 100 && rows <= 32;
+}
+
 template <typename T, bool PE, int NP>
 static int launch_sw(DeviceCtx &c, const b200attn_args *a, int n, const SwParams &p, cudaStream_t st) {
     constexpr bool W = sizeof(T) == 4;
@@ -763,10 +779,9 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
         if (rc != B200ATTN_OK) c->prev_sdtc = false;
         if (rc == B200ATTN_OK) done = true;
         else if (rc != -1) return rc;
-        // What the kernel above takes it keeps (4 heads, 64 x 64, head_d 512 / 2048 9.1 / 11.0 us against 10.4 / 12.8 us streamed, 1 head of
-        // 8192 12.9 against 14.5, 4 heads of 8192 17.9 against 17.8); everything else of these lengths streams where rows allow it:
-        // against the CUDA-core kernels 1.05 (one head, head_d 64) to 4.5 times faster over types, encodings and 1 to 148 heads.
-        if (!done && sw_supported(*c, *a)) {
+        // What the kernel above takes it keeps (4 heads, 64 x 64, head_d 512 / 2048 9.1 / 11.0 us against 9.4 / 11.7 us streamed); of the rest
+        // this takes what it is faster at (sw_slower).
+        if (!done && sw_supported(*c, *a) && !sw_slower(*c, *a)) {
             rc = run_sw(*c, a, 1, rd, base, st);
             if (rc == B200ATTN_OK) done = true;
             else if (rc != -1) return rc;

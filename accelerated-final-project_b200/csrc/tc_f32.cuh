@@ -643,6 +643,13 @@ struct F32Scratch {   // per device, grown on demand
 
 inline bool f32tc_supported(const b200attn_args &a) {
     if (a.len_q <= 64 && a.len_k <= 64) return false;
+    // Few rows on one side are padded to whole tiles here, and with enough blocks for the chip the CUDA-core kernels are done before the
+    // split is (us there / here, fp32: 148 heads, 1 x 65, head_d 512 55 / 94, 1000 heads, 16 x 100, head_d 128 141 / 184, 300 heads, 200 x 8,
+    // head_d 64 46 / 55; bf16: 300 heads, 1 x 128, head_d 80 44 / 52).  Below the lines this is the faster one almost everywhere (64 heads, 1 x 1000,
+    // head_d 128 110 / 74; 148 heads, 300 x 32, head_d 64 51 / 39; still the slower one by up to a quarter: 1000 heads of head_d 16).
+    const long long blocks = (long long)a.batch_sz * a.num_heads * ((a.len_q + 63) / 64) * ((a.head_d + 63) / 64);
+    const int few = a.len_q < a.len_k ? a.len_q : a.len_k, many = a.len_q < a.len_k ? a.len_k : a.len_q;
+    if ((few <= 4 && blocks >= 200) || (few <= 16 && blocks >= 300) || (few <= 32 && many <= 512 && blocks >= 1000)) return false;
     if (a.dtype == B200ATTN_F32) return a.head_d <= 512;
     // 16 bit: the widths up to 256 whose 16-bit kernels would round what the CUDA-core kernels hold in fp32
     if (a.head_d % 8 != 0 || a.head_d > 256 || (a.head_d % 64 == 0 && (a.head_d != 192 || a.len_q <= 64))) return false;

@@ -25,6 +25,19 @@ def test_against_oracle(pkg, cuda, shape):
     assert res["ok"] and res["max_abs"] <= MAX_ABS, (shape, res)
 
 
+@pytest.mark.parametrize("f16", [False, True])
+@pytest.mark.parametrize("shape,path", [((1, 199, 1, 65, 8), "tc_f32"), ((1, 200, 4, 65, 8), "splitd_two_pass"), ((1, 200, 5, 65, 8), "tc_f32"),
+                                        ((1, 150, 65, 16, 8), "splitd_two_pass"), ((1, 150, 65, 17, 8), "tc_f32"), ((1, 250, 100, 32, 72), "splitd_two_pass"),
+                                        ((1, 249, 100, 32, 72), "tc_f32"), ((1, 250, 33, 70, 72), "tc_f32")], ids=str)
+def test_few_rows_on_one_side(pkg, cuda, shape, path, f16):
+    """On either side of the lines between this path and the CUDA-core kernels."""
+    T = [x.astype(np.float16 if f16 else np.float32) for x in ol.make_qkv(*shape, 87, "uniform")]
+    got = pkg.forward(*(to_dev(x, cuda) for x in T))
+    assert pkg.last_path() == path
+    want = ol.attention(*(x.astype(np.float32) for x in T))
+    assert (np.abs(got.float().cpu().numpy() - want) <= MAX_ABS + (np.abs(want) * 2.0 ** -11 if f16 else 0.0)).all()
+
+
 @pytest.mark.parametrize("pe,rd", [(ol.PE_ROPE_INTERLEAVED, 0), (ol.PE_ROPE_INTERLEAVED, 10), (ol.PE_ROPE_HALF, 0), (ol.PE_ROPE_HALF, 12),
                                    (ol.PE_SINUSOIDAL, 0), (ol.PE_ROPE_Q_ONLY, 0)])
 @pytest.mark.parametrize("D", [34, 96])

@@ -54,6 +54,24 @@ def test_fp32(pkg, cuda, shape, pe):
         assert res["max_abs"] <= bound(pe, D), (shape, pe, res)
 
 
+@pytest.mark.parametrize("shape,dtype,pe,path", [
+    ((1, 16, 8, 8, 2048), torch.float32, ol.PE_ROPE_INTERLEAVED, "splitd_fused"), ((1, 16, 8, 9, 2048), torch.float32, ol.PE_ROPE_INTERLEAVED, "splitd_stream"),
+    ((1, 16, 8, 8, 1536), torch.float32, ol.PE_SINUSOIDAL, "splitd_stream"),
+    ((1, 148, 4, 4, 288), torch.float16, ol.PE_SINUSOIDAL, "splitd_stream"), ((1, 148, 16, 16, 128), torch.bfloat16, ol.PE_NONE, "splitd_fused"),
+    ((1, 148, 17, 16, 128), torch.bfloat16, ol.PE_NONE, "splitd_stream"), ((1, 75, 32, 32, 64), torch.float16, ol.PE_NONE, "splitd_fused"),
+    ((1, 75, 32, 33, 64), torch.float16, ol.PE_NONE, "splitd_stream"), ((1, 1, 32, 32, 3232), torch.bfloat16, ol.PE_NONE, "splitd_fused"),
+    ((1, 1, 32, 32, 3200), torch.bfloat16, ol.PE_NONE, "splitd_stream")], ids=str)
+def test_few_rows(pkg, cuda, shape, dtype, pe, path):
+    """On either side of the lines between this kernel and the CUDA-core one."""
+    T = [to_dev(x, cuda).to(dtype) for x in ol.make_qkv(*shape, 89, "uniform")]
+    got = pkg.forward(*T, pe=pe).float().cpu().numpy()
+    if torch.cuda.get_device_properties(cuda).multi_processor_count == 148:
+        assert pkg.last_path() == path
+    want = want_of(*(t.float().cpu().numpy() for t in T), pe)
+    half_ulp = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    assert (np.abs(got - want) <= np.abs(want) * half_ulp + max(bound(pe, shape[-1]), 5e-5)).all()
+
+
 @pytest.mark.parametrize("D,rd", [(36, 0), (64, 6), (200, 34)])
 @pytest.mark.parametrize("pe", [ol.PE_ROPE_INTERLEAVED, ol.PE_ROPE_Q_ONLY])
 def test_partial_rotary(pkg, cuda, D, rd, pe):
