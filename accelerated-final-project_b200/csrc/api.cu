@@ -779,8 +779,9 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
         if (rc != B200ATTN_OK) c->prev_sdtc = false;
         if (rc == B200ATTN_OK) done = true;
         else if (rc != -1) return rc;
-        // What the kernel above takes it keeps (4 heads, 64 x 64, head_d 512 / 2048 9.1 / 11.0 us against 9.4 / 11.7 us streamed); of the rest
-        // this takes what it is faster at (sw_slower).
+        // What the kernel above takes it keeps (4 heads, 64 x 64, head_d 512 / 2048 / 8192 9.3 / 11.2 / 18.0 us against 9.6 / 11.6 / 16.1 us streamed, 16
+        // heads of 1024 13.4 against 12.9: the line is older than the streamed kernel's present form); of the rest this takes what it is faster
+        // at (sw_slower).
         if (!done && sw_supported(*c, *a) && !sw_slower(*c, *a)) {
             rc = run_sw(*c, a, 1, rd, base, st);
             if (rc == B200ATTN_OK) done = true;
@@ -804,7 +805,7 @@ static int forward_device(const b200attn_args *a, bool independent_of_prev = fal
 // but not a group that leaves a third of the SMs out while the others have long slices, nor a call or two left over: those have nothing to
 // overlap with.  So such a run goes out in equal groups or not at all.  Measured, chain / groups: fp32, 64 x 64, 3 entries of 60 heads,
 // head_d 256 (2 + 1) 24 / 37 us; 5 of 32, head_d 512 (4 + 1) 40 / 46 us; 5 of 16 heads, head_d 2048 (a slice a head, 80 CTAs) 69 / 76 us;
-// 2 of 40 heads, head_d 512 22 / 24 us; for: 2 of 16 heads, head_d 512 15.5 / 14.0 us; 4 of 32, head_d 512 36 / 26 us; 16 of 4, head_d 2048
+// 2 of 40 heads, head_d 512 22 / 24 us; for: 2 of 16 heads, head_d 512 15.7 / 12.9 us; 4 of 32, head_d 512 36 / 24 us; 16 of 4, head_d 2048
 // 87 / 43 us.  Other entries (wide slices, encodings) have a launch each otherwise and take the largest group that fills the chip.
 static int batch_group(const b200attn_args *a, int n, int *run) {
     int rd, rd1; float base, base1;

@@ -458,8 +458,6 @@ dec_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     constexpr int kv_stage = nch * DC_KSLAB;
 
     if (threadIdx.x == 0) {
-        mbar_init(&bars.q_full, 1);
-        mbar_init(&bars.q_ready, 4);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bars.k_full[i], 1); mbar_init(&bars.k_ready[i], 4); mbar_init(&bars.k_free[i], 1);
             mbar_init(&bars.v_full[i], 1); mbar_init(&bars.v_free[i], 1);

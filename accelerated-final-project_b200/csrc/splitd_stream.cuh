@@ -17,7 +17,7 @@
 //
 // Precision: operands are cut into bf16 pieces whose sum is exact (fp32 and encoded values three, fp16 two, bf16 one; P three) and
 // the products are collected by their order of magnitude in accumulators of their own (x1 y1 | x1 y2 + x2 y1 | x1 y3 + x2 y2 +
-// x3 y1); what is left out is below 2^-23 of a product, on average 2^-25.  A score accumulator takes 128 columns, the sums over
+// x3 y1); what is left out is below 2^-22 of a product, on average 2^-26 (the first piece is cut off, not rounded: x2 reaches 2^-7 x).  A score accumulator takes 128 columns, the sums over
 // these are added up in fp32 registers: the tensor core cuts a sum off where it does not fit, always towards zero.  Against 64
 // bits (uniform inputs, head_d 2048 to 8192) a hi / lo tf32 form of this kernel erred by 6e-7 to 8e-7, the CUDA-core kernels
 // by 1.1e-7 to 1.8e-7, this form by 0.8e-7 to 1.0e-7.  The encoding and the softmax are fp32 as in splitd.cuh.

@@ -2,8 +2,9 @@
 // head widths that the 16-bit kernels do not take (no multiple of 64; 192 with an encoding).
 //
 // An fp32 value is cut into three bf16 pieces x = x1 + x2 + x3 (8 significant bits each: the sum is exact), and a product
-// a b is taken as a1 b1 + (a1 b2 + a2 b1) + (a1 b3 + a2 b2 + a3 b1): what is left out is below 2^-23 |a b| (about 2^-25 on
-// average).  Six bf16 MMAs cost what three tf32 MMAs on a hi / lo pair cost and keep two more bits.  The leading products
+// a b is taken as a1 b1 + (a1 b2 + a2 b1) + (a1 b3 + a2 b2 + a3 b1): what is left out is below 2^-22 |a b| (2^-26 on average; the
+// first piece is cut off, not rounded, so that a large value does not become an infinity: a2 reaches 2^-7 a).  Values below 2^-110
+// lose low bits, to an absolute error of 2^-134 (of V 2^-103 and 2^-127).  Six bf16 MMAs cost what three tf32 MMAs on a hi / lo pair cost and keep two more bits.  The leading products
 // have an accumulator of their own and are added to the small ones in fp32 by the thread that reads them, and P V starts a
 // fresh accumulator per 64 keys, summed in registers: the chain of roundings at the full magnitude is as short as
 // head_d / 16 and len_k / 64.  (Replaces, for these shapes, the FFMA kernels of splitd.cuh; same mathematics as the
@@ -25,8 +26,8 @@
 //
 // Why two kernels: the three planes of P, Q, K and V of a one-kernel form fill shared memory at head_d 128 and exceed it
 // beyond, while the fp32 scores of the sizes in use stay in the L2.
-// Infinities and NaN: pieces of a non-finite value would turn inf * x into NaN (inf * 0 of a lower piece), so the split
-// kernel marks the call when it meets one and the other two kernels then take plain FFMA loops over the same planes.
+// Infinities and NaN: a non-finite value is its first piece, the others are zero, and the sum of the leading products is the result
+// wherever it is not finite (f3_sum): as in FFMA but for an infinity times a subnormal.
 // Every wait is bounded.
 #pragma once
 

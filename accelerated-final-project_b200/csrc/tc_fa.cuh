@@ -89,7 +89,8 @@ __device__ __forceinline__ void umma_16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
 //     (per key tile the chain softmax -> P V -> Q K^T -> softmax is serial for each query tile)
 //   the same with an issuer per query tile                                                              790
 //   key tiles of 64 keys, two score buffers per query tile, P in tensor memory; one / two issuers   630 / 800
-//     (an MMA of N = 64 costs an issuing thread as much as one of N = 128: 100 to 140 clocks)
+//     (an MMA of N = 64 cost an issuing thread as much as one of N = 128, 100 to 140 clocks: threads chosen by `lane == 0`,
+//     as in every row of this table; an elected one issues them in 49 and 64, and no row has been tried again with it)
 //   this layout, 352 threads, 168 registers per thread                                                 1020
 //   ... with the softmax warpgroups taking over registers of warpgroup 0 (setmaxnreg, no spills)         1110
 //   ... with a quarter / half of the exponentials as a cubic on the FMA pipe instead of ex2      1060 / 940

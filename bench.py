@@ -301,6 +301,7 @@ def fp32_sweep(pkg, torch, dev, pk, with_cpu=True):
         sets = [make_inputs(pkg, torch, cfg, dev, 42 + i) for i in range(nsets)]
         settle(torch)
         cold = min(time_steps(pkg, torch, sets, 0, nsets, nsets if r == 0 else 0) for r in range(3))
+        batch_path = pkg.last_path()   # of the launches that cold_ms is of
         warm = time_steps(pkg, torch, sets[:1], 0, 200, 20)
         serial = min(time_steps(pkg, torch, sets, 0, nsets, 0, flags=pkg.FLAG_NO_OVERLAP) for r in range(2))
         Q, K, V, O = sets[0]
@@ -311,7 +312,7 @@ def fp32_sweep(pkg, torch, dev, pk, with_cpu=True):
         lat = (time.perf_counter() - t0) / 50 * 1e3
         _, _, B, H, Lq, Lk, D, _, _ = CONFIGS[cfg]
         tfl = flops_of(cfg) / cold / 1e9
-        row = {"config": cfg, "shape": [B, H, Lq, Lk, D], "path": pkg.last_path(), "cold_ms": round(cold, 5),
+        row = {"config": cfg, "shape": [B, H, Lq, Lk, D], "path": batch_path, "blocking_call_path": pkg.last_path(), "cold_ms": round(cold, 5),
                "warm_ms": round(warm, 5), "blocking_call_ms": round(lat, 5),
                # the same launches with each one started only after the previous has completed: kernel + launch gap
                "serial_step_us": round(serial * 1e3, 2), "overlap_gain_us": round((serial - cold) * 1e3, 2),

@@ -185,9 +185,9 @@ const char *b200attn_last_error(void);
 /* Name of the kernel path the last successful b200attn_forward_ex on this thread used:
  * "splitd_tc" (fp32, short sequences, tensor cores with error-compensated tf32), "splitd_stream" (short
  * sequences of any type on the tensor cores, streamed slices), "tc_f32" (longer sequences, fp32 with head_d up to 512, 16 bit
- * with head_d up to 256 that is a multiple of 8 and of no use to the 16-bit kernels: three kernels on bf16 pieces of the operands), "splitd_fused" and "splitd_two_pass" (CUDA cores), "tc_wide" (bf16 on the tensor cores: score kernel, then P V kernel),
+ * with head_d a multiple of 8 below 256 but none of 64, or 192 with an encoding: three kernels on bf16 pieces of the operands), "splitd_fused" and "splitd_two_pass" (CUDA cores), "tc_wide" (bf16 on the tensor cores: score kernel, then P V kernel),
  * "tc_fused" (bf16 / fp16, head_d 64, 128, 192 or 256, more than 64 queries: one kernel, scores in tensor
- * memory; an encoding is applied to copies of Q and K first), "tc_bf16" (bf16 on the tensor cores, one-kernel
+ * memory; an encoding is applied to copies of Q and K first, in one launch), "tc_bf16" (bf16 on the tensor cores, one-kernel
  * cluster pipeline) or "tc_decode" (bf16, up to 64 queries against a long K/V: key splits on the tensor cores
  * plus a combine kernel). */
 const char *b200attn_last_path(void);
